@@ -132,6 +132,7 @@ __global__ void __launch_bounds__(256) k_integrate(DevView v, double dt, int rep
             // a hair under skin/2: FP32 rounding can only trigger a rebuild early
             if (v.skin_half2 > 0.0 && d2 > (float)v.skin_half2 * 0.99999f) atomicOr(&v.flags->skin_hit, 1);
         } else {
+            v.uf[s] = box_fraction(S, p[0], p[1], p[2]);
             if (v.skin_half2 > 0.0) {
                 double d2 = 0.0;
 #pragma unroll

@@ -211,6 +211,7 @@ __device__ __forceinline__ void derive_slot(const DevView &v, int s, double x, d
     } else {
         v.qs[s] = qs;
         v.ljd[s] = make_double2(sg, ep);
+        v.uf[s] = box_fraction(S, x, y, z);
         v.xref[s] = x;
         v.xref[v.N + s] = y;
         v.xref[2 * v.N + s] = z;

@@ -14,6 +14,7 @@
 // r^2 < cutoff^2.  The list holds a superset (cutoff + skin, FP32 test with
 // a safety margin); in mixed mode the FP32 r^2 settles every pair except
 // those within 1e-5 relative of the cutoff, which are re-tested in FP64.
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -579,84 +580,270 @@ __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_pairs_mixed
     }
 }
 
-// FP64 form: the same list; every pair in double precision from the FP64
-// positions with the reference's minimum image (NonbondedForce.cpp:548-581).
-template <bool ENERGY>
-__global__ void __launch_bounds__(kHoodWarps * 32) k_pairs_fp64(DevView v) {
+// ---- FP64 form: the same list, every pair once, in double precision from the
+// FP64 positions with the reference's minimum image (NonbondedForce.cpp:548-581).
+//
+// Bound by the FP64 pipe (two lanes per SM and clock on this GPU), so the
+// work is arranged to give that pipe as few instructions as the sum needs:
+//  * a filter on FP32 r^2 from the staged box fractions (integer and FP32
+//    instructions only) drops the list entries beyond the cutoff, and takes
+//    each pair from one of its two lists only (the other atom's force by
+//    atomics, which the FP64 engine's force sums are anyway);
+//  * what passes is compacted into a per-warp queue and evaluated 32 at a
+//    time, so no lane of an FP64 instruction idles;
+//  * comparisons and conversions, FP64 instructions too, are done on the
+//    numbers' bits;
+//  * 1/r by one third-order step from the FP32 reciprocal root, and the Ewald
+//    terms as erf (an entire function of r^2 over r, Taylor rows in a table
+//    that stays in L1) subtracted from the bare Coulomb term: about 40 FP64
+//    instructions per pair, where erfc, exp, sqrt and the divisions took
+//    about 240 per list entry.  23,800 atoms: 5,390 -> 567 us, the FP64 pipe
+//    busy 83% of the kernel's active cycles; 2,700 atoms: 727 -> 96 us.
+// The pair set is decided on the exact r^2 of the reference's list.
+
+constexpr int kWarps64 = 8;
+
+__device__ __forceinline__ long long bits_of(double x) { return __double_as_longlong(x); }
+
+// -x by its sign bit
+__device__ __forceinline__ double negated(double x) {
+    return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
+}
+
+// min_image() with |d| > L/2 compared as integers (the order of non-negative
+// doubles), and no FP64 addition issued for a warp none of whose lanes shifts.
+__device__ __forceinline__ double min_image_bits(double d, double L, double halfL) {
+    const long long b = __double_as_longlong(d);
+    const bool far = (b & 0x7fffffffffffffffLL) > __double_as_longlong(halfL);
+    if (__any_sync(__activemask(), far)) {
+        if (far) d += b < 0 ? L : -L;
+    }
+    return d;
+}
+
+template <bool ENERGY, bool SW>
+struct Pairs64 {
+    const DevView &v;
+    const SysDev &S;
+    const double L0, L1, L2, h0, h1, h2, cut2, alpha2, alpha3, sw_dist, sw_inv;
+    const long long near_bits;  // r^2 from here on: too close to the cutoff for a fused r^2 to decide
+    const float a2f;
+    double fx = 0, fy = 0, fz = 0, ec = 0, ev = 0;
+    int cur = -1;  // the atom the warp's sums fx, fy, fz belong to
+
+    __device__ Pairs64(const DevView &v_, const SysDev &S_)
+        : v(v_), S(S_), L0(S_.L[0]), L1(S_.L[1]), L2(S_.L[2]), h0(S_.halfL[0]), h1(S_.halfL[1]), h2(S_.halfL[2]),
+          cut2(S_.cut2), alpha2(S_.alpha2), alpha3(S_.alpha3), sw_dist(S_.sw_dist),
+          sw_inv(SW ? 1.0 / (S_.cutoff - S_.sw_dist) : 0.0), near_bits(bits_of(S_.cut2 * (1.0 - 1e-14))),
+          a2f((float)(S_.alpha2 * kBoysPerUnit)) {}
+
+    // the pair (i, j): j's force by atomics; i's into the warp's sums where i
+    // is `cur`, by atomics otherwise
+    __device__ __forceinline__ void pair(int i, int j) {
+        // d = p_j - p_i; near the cutoff r^2 is formed again as the list
+        // decides (exact_r2)
+        const double dx = min_image_bits(__dsub_rn(v.x[j], v.x[i]), L0, h0);
+        const double dy = min_image_bits(__dsub_rn(v.y[j], v.y[i]), L1, h1);
+        const double dz = min_image_bits(__dsub_rn(v.z[j], v.z[i]), L2, h2);
+        const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+        const long long rb = __double_as_longlong(r2);
+        if (rb >= near_bits) {
+            const double x2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+            if (!(x2 < cut2)) return;
+        }
+        // r^2 to FP32 by its bits (truncated), 1/r from the FP32 estimate y
+        // (e = 1 - r^2 y^2 below 2^-20): y (1 + e/2 + 3 e^2 / 8), error e^3
+        const int hi = (int)(rb >> 32);
+        const float r2f = __int_as_float(((hi - 0x38000000) << 3) | (int)((unsigned)rb >> 29));
+        double rinv;
+        if (hi > 0x39000000 && hi < 0x46000000) {
+            const unsigned yb = __float_as_uint(fast_rsqrt(r2f));
+            const double y = __hiloint2double((int)((yb >> 3) + 0x38000000u), (int)(yb << 29));
+            const double e = fma(-(r2 * y), y, 1.0);
+            rinv = fma(y * e, fma(e, 0.375, 0.5), y);
+        } else {
+            rinv = 1.0 / sqrt(r2);  // outside FP32's range (coinciding atoms among them)
+        }
+        const double rinv2 = rinv * rinv;
+        const double2 li = v.ljd[i], lj = v.ljd[j];
+        const double qq = v.qs[i] * v.qs[j];
+        const double sr = (li.x + lj.x) * rinv;
+        const double s2 = sr * sr;
+        const double s6 = s2 * s2 * s2;
+        const double es6 = li.y * lj.y * s6;
+        double vdw = es6 * fma(12.0, s6, -6.0);  // times 1/r^2 below
+        double evdw = (ENERGY || SW) ? fma(es6, s6, -es6) : 0.0;
+        if (SW && S.use_switch) {
+            const double r = r2 * rinv;
+            if (r > sw_dist) {
+                const double t = (r - sw_dist) * sw_inv;
+                const double sw = 1 + t * t * t * (-10 + t * (15 - t * 6));
+                const double dsw = t * t * (-30 + t * (60 - t * 30)) * sw_inv;
+                vdw = sw * vdw - evdw * dsw * r;
+                evdw *= sw;
+            }
+        }
+        // Ewald: erfc/r^3 + ... = 1/r^3 - alpha^3 H(s); erfc/r = 1/r - alpha E(s)
+        const int row = (int)(r2f * a2f);
+        double coul = 0.0, ecoul = 0.0;
+        if (row < kBoysRows) {
+            const double2 *c = reinterpret_cast<const double2 *>(v.boys) + (kBoysRow / 2) * max(row, 0);
+            const double2 c67 = __ldg(c + 3), c45 = __ldg(c + 2), c23 = __ldg(c + 1), c01 = __ldg(c);
+            const double t = fma(r2, alpha2, -c67.y);
+            double p = fma(c67.x, t, c45.y);
+            p = fma(p, t, c45.x);
+            p = fma(p, t, c23.y);
+            p = fma(p, t, c23.x);
+            p = fma(p, t, c01.y);
+            p = fma(p, t, c01.x);
+            coul = fma(-alpha3, p, rinv * rinv2);
+            if (ENERGY) {
+                const double2 *d = c + (kBoysRow / 2) * kBoysRows;
+                const double2 d67 = __ldg(d + 3), d45 = __ldg(d + 2), d23 = __ldg(d + 1), d01 = __ldg(d);
+                p = fma(d67.x, t, d45.y);
+                p = fma(p, t, d45.x);
+                p = fma(p, t, d23.y);
+                p = fma(p, t, d23.x);
+                p = fma(p, t, d01.y);
+                p = fma(p, t, d01.x);
+                ecoul = fma(-S.alpha, p, rinv);
+            }
+        }
+        const double dEdR = fma(qq, coul, vdw * rinv2);
+        const double gx = dx * dEdR, gy = dy * dEdR, gz = dz * dEdR;  // on j
+        double *ax = static_cast<double *>(v.fx), *ay = static_cast<double *>(v.fy), *az = static_cast<double *>(v.fz);
+        atomicAdd(ax + j, gx);
+        atomicAdd(ay + j, gy);
+        atomicAdd(az + j, gz);
+        if (i == cur) {
+            fx += gx;
+            fy += gy;
+            fz += gz;
+        } else {
+            atomicAdd(ax + i, negated(gx));
+            atomicAdd(ay + i, negated(gy));
+            atomicAdd(az + i, negated(gz));
+        }
+        if (ENERGY) {
+            ec = fma(qq, ecoul, ec);
+            ev += evdw;
+        }
+    }
+
+    // the warp's sums to atom `cur`: three sums over 32 lanes in six
+    // additions (x and y share lanes from the first step, z from the second)
+    __device__ __forceinline__ void flush(int lane) {
+        const unsigned full = 0xffffffffu;
+        const bool up16 = lane & 16, up8 = lane & 8;
+        double a = up16 ? fy : fx;
+        a += __shfl_xor_sync(full, up16 ? fx : fy, 16);  // x in lanes 0-15, y in 16-31
+        double b = fz + __shfl_xor_sync(full, fz, 16);   // z, both halves alike
+        double c = up8 ? b : a;
+        c += __shfl_xor_sync(full, up8 ? a : b, 8);      // bit 3 clear: x or y; set: z
+        c += __shfl_xor_sync(full, c, 4);
+        c += __shfl_xor_sync(full, c, 2);
+        c += __shfl_xor_sync(full, c, 1);
+        double *f = static_cast<double *>(up8 ? v.fz : (up16 ? v.fy : v.fx));
+        if ((lane & 7) == 0 && lane != 24) atomicAdd(f + cur, negated(c));
+        fx = fy = fz = 0.0;
+    }
+};
+
+template <bool ENERGY, bool SW>
+__global__ void __launch_bounds__(kWarps64 * 32, 2) k_pairs_fp64(DevView v) {
     extern __shared__ __align__(16) unsigned char smem[];
+    const unsigned full = 0xffffffffu;
     CellGroup G = v.groups[blockIdx.x];
-    int a0 = v.cell_start[G.cell], a1 = v.cell_start[G.cell + G.ncell];
+    const int a0 = v.cell_start[G.cell], a1 = v.cell_start[G.cell + G.ncell];
     if (a0 == a1) return;
     const SysDev &S = v.sys[G.sys];
     if (!S.nb_on) return;
-    HoodSpan *spans = reinterpret_cast<HoodSpan *>(smem);
-    int *s_n = reinterpret_cast<int *>(spans + kMaxSpans);
-    int n = hood_setup(v, S, v.cell3[a0], G.ncell, spans, s_n, nullptr);
-    if (n > v.hood_cap || s_n[1] > kMaxSpans) {
+    // tile: box fractions and the slot of each atom of the neighbourhood
+    int4 *s_u = reinterpret_cast<int4 *>(smem);
+    HoodSpan *spans = reinterpret_cast<HoodSpan *>(s_u + v.hood_cap);
+    __shared__ int2 s_queue[kWarps64][64];
+    __shared__ int2 s_nn;
+    __shared__ int s_next;
+    {
+        const int *src = v.gspan + (size_t)blockIdx.x * kGroupSpanWords;
+        int *dst = reinterpret_cast<int *>(spans);
+        for (int e = threadIdx.x; e < kGroupSpanWords; e += blockDim.x) dst[e] = src[e];
+        if (threadIdx.x == 0) {
+            s_nn = v.gspan_n[blockIdx.x];
+            s_next = 0;
+        }
+    }
+    __syncthreads();
+    const int n = s_nn.x, nsp = s_nn.y;
+    if (n > v.hood_cap || nsp > kMaxSpans) {
         if (threadIdx.x == 0) atomicOr(&v.flags->error, ERR_NLIST_OVERFLOW);
         return;
     }
-    int nsp = s_n[1];
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    double ec = 0, ev = 0;
-    for (int i = a0 + warp; i < a1; i += nw) {
-        double xi = v.x[i], yi = v.y[i], zi = v.z[i];
-        double qi = v.qs[i];
-        double2 li = v.ljd[i];
-        int cnt = v.ncount[i];
-        const uint16_t *lst = v.nl16 + (size_t)i * v.stride;
-        double fx = 0, fy = 0, fz = 0;
-        for (int k = lane; k < cnt; k += 32) {
-            int j = hood_slot(spans, nsp, lst[list_pos(k)] >> kEntryShift);
-            if (!(exact_r2(v, S, i, j) < S.cut2)) continue;
-            // deltaR = minimumImageVector(p_i, p_j) (NonbondedForce.cpp:548)
-            double dx = min_image(xi - v.x[j], S.L[0], S.halfL[0]);
-            double dy = min_image(yi - v.y[j], S.L[1], S.halfL[1]);
-            double dz = min_image(zi - v.z[j], S.L[2], S.halfL[2]);
-            double r = sqrt(dx * dx + dy * dy + dz * dz);
-            double rinv = 1.0 / r;
-            double sw = 1.0, dsw = 0.0;
-            if (S.use_switch && r > S.sw_dist) {
-                double t = (r - S.sw_dist) / (S.cutoff - S.sw_dist);
-                sw = 1 + t * t * t * (-10 + t * (15 - t * 6));
-                dsw = t * t * (-30 + t * (60 - t * 30)) / (S.cutoff - S.sw_dist);
-            }
-            double xa = S.alpha * r;
-            double qq = qi * v.qs[j];
-            double erfcv = erfc(xa);
-            double dEdR = qq * rinv * rinv * rinv * (erfcv + 2 * xa * exp(-xa * xa) / kSqrtPi);
-            double2 lj = v.ljd[j];
-            double sg = li.x + lj.x;
-            double s2 = sg * rinv;
-            s2 *= s2;
-            double s6 = s2 * s2 * s2;
-            double eps = li.y * lj.y;
-            dEdR += sw * eps * (12.0 * s6 - 6.0) * s6 * rinv * rinv;
-            double evdw = eps * (s6 - 1.0) * s6;
-            if (S.use_switch) {
-                dEdR -= evdw * dsw * rinv;
-                evdw *= sw;
-            }
-            fx += dx * dEdR;
-            fy += dy * dEdR;
-            fz += dz * dEdR;
-            if (ENERGY) {
-                ec += qq * rinv * erfcv;
-                ev += evdw;
-            }
-        }
-        fx = warp_sum(fx);
-        fy = warp_sum(fy);
-        fz = warp_sum(fz);
-        if (lane == 0) {
-            atomicAdd(static_cast<double *>(v.fx) + i, fx);
-            atomicAdd(static_cast<double *>(v.fy) + i, fy);
-            atomicAdd(static_cast<double *>(v.fz) + i, fz);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = kWarps64;
+    for (int sp = warp; sp < nsp; sp += nw) {
+        const HoodSpan h = spans[sp];
+        for (int t = lane; t < h.count; t += 32) {
+            int4 u = v.uf[h.start + t];
+            u.w = h.start + t;
+            s_u[h.offset + t] = u;
         }
     }
+    __syncthreads();
+    Pairs64<ENERGY, SW> P(v, S);
+    const float ux = S.u2nm[0], uy = S.u2nm[1], uz = S.u2nm[2], pre = S.cut2f_pre;
+    int2 *queue = s_queue[warp];
+    const unsigned lt = (1u << lane) - 1u;
+    int head = 0, tail = 0;  // the queue holds entries head .. tail - 1 (at most 63), entry k at k & 63
+    // a unit of work: the even or the odd chunks of one atom's list, taken by
+    // the next warp that is free
+    for (;;) {
+        int t = lane == 0 ? atomicAdd(&s_next, 1) : 0;
+        t = __shfl_sync(full, t, 0) * gridDim.y + blockIdx.y;
+        const int i = a0 + (t >> 1);
+        if (i >= a1) break;
+        const int4 ui = v.uf[i];
+        const int cnt = v.ncount[i];
+        const uint4 *lst4 = reinterpret_cast<const uint4 *>(v.nl16 + (size_t)i * v.stride) + lane;
+        P.cur = i;
+        for (int c0 = 256 * (t & 1); c0 < cnt; c0 += 512) {
+            const uint4 w4 = __ldg(lst4 + c0 / 8);
+            const uint32_t wds[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (c0 + 32 * u >= cnt) break;  // warp-uniform
+                const bool valid = c0 + 32 * u + lane < cnt;
+                const unsigned e = (wds[u >> 1] >> (16 * (u & 1))) & 0xffffu;
+                const int4 uj = s_u[valid ? e >> kEntryShift : 0];
+                const float dx = (float)(uj.x - ui.x) * ux, dy = (float)(uj.y - ui.y) * uy,
+                            dz = (float)(uj.z - ui.z) * uz;
+                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                const int j = uj.w;
+                // each pair from one of its two lists, half of them either way
+                const bool mine = (((i ^ j) & 1) != 0) == (i < j);
+                const unsigned m = __ballot_sync(full, valid && mine && r2 < pre);
+                if ((m >> lane) & 1u) queue[(tail + __popc(m & lt)) & 63] = make_int2(i, j);
+                tail += __popc(m);
+                if (tail - head >= 32) {
+                    __syncwarp();
+                    const int2 p = queue[(head + lane) & 63];
+                    P.pair(p.x, p.y);
+                    head += 32;
+                    __syncwarp();
+                }
+            }
+        }
+        P.flush(lane);
+    }
+    P.cur = -1;
+    __syncwarp();
+    if (head + lane < tail) {
+        const int2 p = queue[(head + lane) & 63];
+        P.pair(p.x, p.y);
+    }
+    __syncwarp();
     if (ENERGY) {
-        energy_add(v.E, G.sys, E_COUL, 0.5 * ec);
-        energy_add(v.E, G.sys, E_VDW, 0.5 * ev);
+        energy_add(v.E, G.sys, E_COUL, P.ec);
+        energy_add(v.E, G.sys, E_VDW, P.ev);
     }
 }
 
@@ -700,9 +887,8 @@ static size_t smem_build(int cap, int warps) {
     return (size_t)cap * sizeof(float4) + (size_t)warps * 512 * sizeof(uint16_t) +
            25 * (kRowCells + 1) * sizeof(int) + tail_bytes();
 }
-static size_t smem_pairs(int cap, int mixed) {
-    return mixed ? (size_t)cap * (sizeof(float4) + sizeof(float2)) + tail_bytes() : tail_bytes();
-}
+static size_t smem_pairs(int cap) { return (size_t)cap * (sizeof(float4) + sizeof(float2)) + tail_bytes(); }
+static size_t smem_pairs64(int cap) { return (size_t)cap * sizeof(int4) + tail_bytes(); }
 // static shared memory of the tile kernels (displacement table and counts)
 constexpr size_t kTileStatic = 25 * kRowCells * sizeof(float4) + 16;
 
@@ -712,7 +898,7 @@ constexpr size_t kTileStatic = 25 * kRowCells * sizeof(float4) + 16;
 // neighbourhoods -- one-cell groups of large cells -- need the latter.)
 static bool wide(size_t dynamic_smem) { return 2 * (dynamic_smem + kTileStatic + 1024) > 228 * 1024; }
 static int build_warps(int cap) { return wide(smem_build(cap, kHoodWarps)) ? 2 * kHoodWarps : kHoodWarps; }
-static int pair_warps(int cap) { return wide(smem_pairs(cap, 1)) ? 2 * kHoodWarps : kHoodWarps; }
+static int pair_warps(int cap) { return wide(smem_pairs(cap)) ? 2 * kHoodWarps : kHoodWarps; }
 
 template <int W>
 static void set_pairs_smem(int m) {
@@ -727,12 +913,13 @@ static void set_pairs_smem(int m) {
 // with a smaller neighbourhood cannot lower it under another one.
 void tiles_set_smem(int cap) {
     static std::mutex mu;
-    static int seen_build[2][kMaxSmemDevices] = {}, seen_pairs[2][kMaxSmemDevices] = {};
+    static int seen_build[2][kMaxSmemDevices] = {}, seen_pairs[2][kMaxSmemDevices] = {},
+               seen_pairs64[kMaxSmemDevices] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= kMaxSmemDevices) dev = 0;
     const int bw = build_warps(cap), pw = pair_warps(cap);
-    const int b = (int)smem_build(cap, bw), m = (int)smem_pairs(cap, 1);
+    const int b = (int)smem_build(cap, bw), m = (int)smem_pairs(cap), d = (int)smem_pairs64(cap);
     const int bi = bw == kHoodWarps ? 0 : 1, pi = pw == kHoodWarps ? 0 : 1;
     std::lock_guard<std::mutex> lock(mu);
     // launches up to 48 KB need no attribute
@@ -750,6 +937,13 @@ void tiles_set_smem(int cap) {
             set_pairs_smem<kHoodWarps>(m);
         seen_pairs[pi][dev] = m;
     }
+    if (d > 48 * 1024 && d > seen_pairs64[dev]) {
+        cudaFuncSetAttribute(k_pairs_fp64<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, d);
+        cudaFuncSetAttribute(k_pairs_fp64<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, d);
+        cudaFuncSetAttribute(k_pairs_fp64<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, d);
+        cudaFuncSetAttribute(k_pairs_fp64<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, d);
+        seen_pairs64[dev] = d;
+    }
 }
 
 void launch_build(const DevView &v, cudaStream_t st) {
@@ -764,7 +958,7 @@ void launch_build(const DevView &v, cudaStream_t st) {
 template <int W>
 static void launch_pairs_mixed(const DevView &v, int energy, cudaStream_t st) {
     const int g = v.ngroups, t = W * 32;
-    const size_t sm = smem_pairs(v.hood_cap, 1);
+    const size_t sm = smem_pairs(v.hood_cap);
     if (v.any_switch) {
         if (energy)
             k_pairs_mixed<true, true, W><<<g, t, sm, st>>>(v);
@@ -787,12 +981,35 @@ void launch_pairs(const DevView &v, int energy, cudaStream_t st) {
             launch_pairs_mixed<2 * kHoodWarps>(v, energy, st);
         return;
     }
-    int g = v.ngroups, t = kHoodWarps * 32;
-    size_t sm = smem_pairs(v.hood_cap, 0);
-    if (energy)
-        k_pairs_fp64<true><<<g, t, sm, st>>>(v);
-    else
-        k_pairs_fp64<false><<<g, t, sm, st>>>(v);
+    // A group's atoms may be dealt to several blocks, each staging the
+    // neighbourhood for itself: as many blocks as make the busiest SM's share
+    // of the atoms least (the pipe that bounds the kernel belongs to the SM,
+    // so its time is its atoms, however many blocks hold them).  23,800
+    // atoms, 484 groups on 152 SMs: 652 us with one block per group, 567 so.
+    const int per = (v.N + v.ngroups - 1) / v.ngroups;
+    int parts = 1, best = 1 << 30;
+    for (int p = 1; p <= (per + kWarps64 - 1) / kWarps64; ++p) {
+        const long long rounds = ((long long)v.ngroups * p + 151) / 152;
+        const int cost = (int)std::min<long long>(rounds * ((per + p - 1) / p), 1 << 29);
+        if (cost <= best) {
+            best = cost;
+            parts = p;
+        }
+    }
+    const dim3 g(v.ngroups, parts);
+    const int t = kWarps64 * 32;
+    const size_t sm = smem_pairs64(v.hood_cap);
+    if (v.any_switch) {
+        if (energy)
+            k_pairs_fp64<true, true><<<g, t, sm, st>>>(v);
+        else
+            k_pairs_fp64<false, true><<<g, t, sm, st>>>(v);
+    } else {
+        if (energy)
+            k_pairs_fp64<true, false><<<g, t, sm, st>>>(v);
+        else
+            k_pairs_fp64<false, false><<<g, t, sm, st>>>(v);
+    }
 }
 
 long long launch_collect_pairs(const DevView &v, int sys, int *out_pairs, long long cap, cudaStream_t st) {

@@ -93,7 +93,18 @@ struct SysDev {
     // order-preserving integer keys (dkey) of the box corners, for the
     // update's wrap test without FP64 comparisons
     long long lbkey[3], ubkey[3];
+    // FP64 pair kernel: alpha^2 and alpha^3, and its FP32 distance filter on
+    // box fractions in 2^-32 (DevView::uf): nm per unit, and the cutoff^2
+    // raised by more than the filter's rounding
+    double alpha2, alpha3;
+    float u2nm[3], cut2f_pre;
 };
+
+// Taylor rows of the FP64 pair kernel's Ewald terms: row k covers s =
+// (alpha r)^2 in [k, k + 1) / kBoysPerUnit; beyond kBoysMax erfc(sqrt s) is
+// below 4e-19, half an ulp of the bare Coulomb term it is a share of.
+constexpr int kBoysPerUnit = 32, kBoysMax = 40, kBoysRows = kBoysPerUnit * kBoysMax;
+constexpr int kBoysRow = 8;  // doubles per row: seven coefficients, the centre
 
 // Flags word layout in device memory.
 struct Flags {
@@ -208,6 +219,20 @@ __device__ __forceinline__ float min_image_f(double d, double L, float halfLf) {
     else if (f < -halfLf)
         f = (float)(d + L);
     return f;
+}
+
+// A position as fractions of the box edges modulo 1, in units of 2^-32: the
+// wrap-around difference of two such words is the minimum image.
+__device__ __forceinline__ int4 box_fraction(const SysDev &S, double x, double y, double z) {
+    const double p[3] = {x, y, z};
+    int u[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        double t = (p[d] - S.lb[d]) * S.invL[d];
+        t -= floor(t);
+        u[d] = (int)__double2uint_rz(t * 4294967296.0);
+    }
+    return make_int4(u[0], u[1], u[2], 0);
 }
 
 template <typename T>

@@ -211,6 +211,45 @@ static void bspline_moduli(int K, std::vector<double> &mod) {
 // buffer, then a merge with the atom's sorted exception partners.  The
 // creation builds the same sets on the device (k_exclusions_build.cu); this
 // host form serves a batch with a row longer than the device search holds.
+// Taylor rows of the FP64 pair kernel's Ewald terms (nxm_common.cuh:
+// kBoysRows), made once per process.  With s = (alpha r)^2,
+//   erf(alpha r) / (alpha r)                                = 2/sqrt(pi) F_0(s)
+//   (erf(alpha r) - 2 alpha r e^-s / sqrt(pi)) / (alpha r)^3 = 4/sqrt(pi) F_1(s)
+// where F_m(s) = integral_0^1 t^2m e^(-s t^2) dt (the Boys functions), and
+// dF_m/ds = -F_(m+1) gives the coefficients about a row's centre: degree 6
+// over half a row (1/64) leaves (1/64)^7 / 7! / 17 < 1e-17.  F_m comes from
+// its series at the highest order, whose terms are all positive, and from
+// there by downward recursion, which is stable: each value within a few ulp.
+static const std::vector<double> &boys_rows() {
+    static const std::vector<double> rows = [] {
+        std::vector<double> t((size_t)2 * kBoysRows * kBoysRow);
+        for (int k = 0; k < kBoysRows; ++k) {
+            const double s = (k + 0.5) / kBoysPerUnit, ex = std::exp(-s);
+            constexpr int M = kBoysRow - 1;
+            double F[M + 1];
+            double term = 1.0 / (2 * M + 1), sum = term;
+            for (int j = 1; term > sum * 1e-18; ++j) {
+                term *= 2 * s / (2 * M + 2 * j + 1);
+                sum += term;
+            }
+            F[M] = ex * sum;
+            for (int m = M - 1; m >= 0; --m) F[m] = (2 * s * F[m + 1] + ex) / (2 * m + 1);
+            for (int which = 0; which < 2; ++which) {
+                // which 0: the force's rows (F_1), 1: the energy's (F_0)
+                double *row = &t[((size_t)which * kBoysRows + k) * kBoysRow];
+                double f = (which ? 2.0 : 4.0) / kSqrtPi;
+                for (int c = 0; c < kBoysRow - 1; ++c) {
+                    row[c] = f * F[c + (which ? 0 : 1)];
+                    f /= -(c + 1);
+                }
+                row[kBoysRow - 1] = s;
+            }
+        }
+        return t;
+    }();
+    return rows;
+}
+
 static std::string exclusion_rows(const HostSystem &s, int off, std::vector<int> &eoff, std::vector<int> &elst,
                                   std::vector<int2> &ex_pairs) {
     const int n = s.n;
@@ -616,6 +655,19 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
         D.ex2c = (float)(-H.alpha * H.alpha * 1.4426950408889634);  // log2(e)
         D.a04 = (float)(0.4 * H.alpha);
         D.k2a = (float)(2.0 * H.alpha / kSqrtPi);
+        D.alpha2 = H.alpha * H.alpha;
+        D.alpha3 = D.alpha2 * H.alpha;
+        {
+            // relative rounding of the filter's FP32 r^2 (< 1e-6) and its
+            // grain: each displacement is within 2 units of 2^-32 of the edge
+            double grain = 0.0;
+            for (int d = 0; d < 3; ++d) {
+                D.u2nm[d] = (float)(H.L[d] * 0x1p-32);
+                grain += 2.0 * H.L[d] * 0x1p-32;
+            }
+            const double reach = h.cutoff + grain;
+            D.cut2f_pre = (float)(reach * reach * (1.0 + 1e-5));
+        }
         for (int d = 0; d < 3; ++d) D.csf[d] = (float)D.cs[d];
         for (int d = 0; d < 3; ++d) {
             D.L40[d] = fix40(H.L[d]);
@@ -802,6 +854,7 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
     } else {
         v_.qs = dalloc<double>(N_);
         v_.ljd = dalloc<double2>(N_);
+        v_.uf = dalloc<int4>(N_);
         v_.fx = dalloc<double>(N_);
         v_.fy = dalloc<double>(N_);
         v_.fz = dalloc<double>(N_);
@@ -890,6 +943,14 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
     }
     up(v_.tmp, positions, sizeof(double) * 3 * (size_t)N_);
     launch_init_atoms(v_, v_.tmp, kst());
+
+    double *boys = nullptr;
+    if (!mixed_) {
+        const std::vector<double> &t = boys_rows();
+        boys = dalloc<double>(t.size());
+        up(boys, t.data(), sizeof(double) * t.size());
+        v_.boys = boys;
+    }
 
     // cell-image displacement table: code ((ox+2)*5 + (oy+2))*12 + (oz+2) -> -(o . cs),
     // o relative to the first cell of a group (oz from -2 to kMaxGroupCells + 1)

@@ -36,6 +36,8 @@ struct DevView {
     float2 *ljf;         // mixed: sigma/2, 2 sqrt(eps)
     double *qs;          // fp64: q * sqrt(ke)
     double2 *ljd;        // fp64: sigma/2, 2 sqrt(eps)
+    int4 *uf;            // fp64: box fraction (p - lb) / L of x, y, z modulo 1, in 2^-32 (the pair kernel's filter)
+    const double *boys;  // fp64: Taylor rows of the Ewald terms: [kBoysRows][kBoysRow] force, then energy
     int *cell3;          // slot -> packed cell coordinates (x | y<<10 | z<<20)
     // force accumulators (long long in mixed mode, double in fp64 mode)
     void *fx, *fy, *fz;
