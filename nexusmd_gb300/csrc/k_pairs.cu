@@ -39,21 +39,6 @@ __device__ __forceinline__ void offset_in_cell(const DevView &v, const SysDev &S
     for (int d = 0; d < 3; ++d) o[d] = (float)min_image(p[d] - (S.lb[d] + c[d] * S.cs[d]), S.L[d], S.halfL[d]);
 }
 
-// Atom i's position in the frame of the group's first cell.
-__device__ __forceinline__ void i_in_group_frame(const DevView &v, const SysDev &S, int i, int cz_first, float p[3]) {
-    int c3 = v.cell3[i];
-    float gz = (float)wrap_once(((c3 >> 20) & 1023) - cz_first, S.nc[2]) * S.csf[2];
-    if (v.mixed) {
-        float4 q = v.pf[i];
-        p[0] = q.x;
-        p[1] = q.y;
-        p[2] = q.z + gz;
-    } else {
-        offset_in_cell(v, S, i, c3, p);
-        p[2] += gz;
-    }
-}
-
 // This system's cell-image displacements (v.dtab: code r * kRowCells +
 // oz + 2 -> -(ox, oy, oz) * cell edge) copied into shared memory by the
 // threads outside warp 0 while warp 0 enumerates the neighbourhood; read
@@ -124,24 +109,53 @@ __device__ void stage(const DevView &v, const SysDev &S, float4 *s_q, float2 *s_
     __syncthreads();
 }
 
-// List layout: each 256-entry chunk of an atom's list is stored transposed,
-// entry p of the chunk at position 8 * (p mod 32) + p / 32, so that lane L
-// of a warp fetches entries L, L+32, ..., L+224 with one 16-byte load.
-// An entry holds 8 times the tile index (the byte offset of the atom's LJ
-// pair in the pair kernel's staged tile; tile indices stay below 8,192).
+// Lists.  One list serves two atoms of a cell, the pair that k_cellsort put
+// together (near neighbours, most often bonded ones; pair_first and
+// DevView::ipair): the union of their neighbours, of which 12% belong to one
+// of them only.  A list's 256-entry chunks are stored transposed, entry p of
+// a chunk at position 8 * (p mod 32) + p / 32, so that lane L of a warp
+// fetches entries L, L+32, ..., L+224 with one 16-byte load.  An entry holds
+// 8 times the tile index (the byte offset of the atom's LJ pair in the pair
+// kernel's staged tile; tile indices stay below 8,192) and in its low bits
+// which of the two atoms it is excluded from (1: the first, 2: the second;
+// from both: no entry); such entries come last.  The list ends with entries
+// of the tile's spare place (an atom beyond every cutoff) up to a multiple of
+// 32, so that the walk needs no range check.
 __device__ __forceinline__ int list_pos(int p) { return (p & ~255) | ((p & 31) << 3) | ((p >> 5) & 7); }
 constexpr int kEntryShift = 3;
+constexpr int kTileSpare = 32;  // places behind a staged tile's capacity, the first of them the spare one
+
+// Shared memory by 32-bit addresses: base plus entry is an address as it is.
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ float4 lds128(unsigned a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float2 lds64(unsigned a) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ int lds32(unsigned a) {
+    int v;
+    asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts32(unsigned a, int v) {
+    asm volatile("st.shared.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void sts16(unsigned a, int v) {
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((short)v) : "memory");
+}
+
+// The list of pair q in memory.
+__device__ __forceinline__ uint16_t *pair_list(const DevView &v, int q) {
+    return v.nl16 + (size_t)q * pair_stride(v.stride);
+}
 
 // ------------------------------------------------------------------ build
 
-// Each warp takes atoms of the group; every staged atom within the list
-// radius that is not i itself and not excluded is appended to i's list as
-// its 16-bit tile index (ballot compaction: deterministic order).  An atom
-// scans only the rows of the neighbourhood its list sphere reaches, and in
-// each row (z-sorted: k_cellsort orders every cell by z) only the atoms
-// within the z extent the sphere has over that row, found by binary search
-// (0.01 nm margin), in tile order: the list is the one a scan of the whole
-// tile gives.
 // Stores one 256-entry list chunk held in order in shared memory as the list
 // layout wants it: lane l writes 16 bytes, entries l + 32 q for q = 0..7.
 __device__ __forceinline__ void store_chunk(uint16_t *dst, const uint16_t *src, int lane) {
@@ -151,9 +165,58 @@ __device__ __forceinline__ void store_chunk(uint16_t *dst, const uint16_t *src, 
     reinterpret_cast<uint4 *>(dst)[lane] = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// An atom of a pair, for the build: its tile position, original index and
+// exclusion partners (the first 32 in shared memory at `list`).
+struct BuildAtom {
+    float x, y, z;
+    int oi, e0, ne, lo;
+    unsigned win, list;
+    __device__ __forceinline__ void load(const DevView &v, float4 q, unsigned list_, int lane) {
+        x = q.x;
+        y = q.y;
+        z = q.z;
+        oi = __float_as_int(q.w);
+        list = list_;
+        e0 = v.excl_off[oi];
+        ne = v.excl_off[oi + 1] - e0;
+        if (lane < ne) sts32(list + 4 * lane, v.excl_lst[e0 + lane]);
+        // Index window [lo, lo + win] of the atom itself and its exclusion
+        // partners (rows ascending): a candidate outside it needs no
+        // membership test.  The atom is left out by its index too, so every
+        // image of it is (the far one lies beyond the list radius anyway).
+        lo = ne ? min(v.excl_lst[e0], oi) : oi;
+        win = (unsigned)((ne ? max(v.excl_lst[e0 + ne - 1], oi) : oi) - lo);
+    }
+    __device__ __forceinline__ bool excluded(const DevView &v, int oj) const {
+        bool ex = oj == oi;
+        for (int e = 0; e < min(ne, 32); ++e) ex |= lds32(list + 4 * e) == oj;
+        for (int e = 32; e < ne; ++e) ex |= v.excl_lst[e0 + e] == oj;
+        return ex;
+    }
+    __device__ __forceinline__ float r2(const float4 &q) const {
+        const float dx = x - q.x, dy = y - q.y, dz = z - q.z;
+        return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+    }
+};
+
+// Each warp takes pairs of the group; every staged atom within the list
+// radius of one of the two and not excluded from it is appended to the
+// pair's list (ballot compaction: deterministic order).  A pair scans only
+// the rows of the neighbourhood its list spheres reach, and in each row
+// (z-sorted: k_cellsort orders every cell by z) only the atoms within the z
+// extent the spheres have over that row, found by binary search (0.01 nm
+// margin), in tile order: the list is the one a scan of the whole tile gives.
+//
+// Bound by instruction issue: a warp tests 32 candidates against both atoms
+// with one load of each candidate and one compaction, so an atom costs about
+// two thirds of what a list of its own does, and half the list traffic.
+// 94,100 atoms: 312 us with a list per atom, 241 so (257 -> 179 M warp
+// instructions); 473,400: 1,730 -> 1,330.
+//
 // W warps per block: 16 (two blocks per SM) or, when two blocks' shared
 // memory does not fit on an SM, 32 (one block per SM, the same 32 warps).
-template <int W>
+constexpr int kKeep = 64, kBuildWarpWords = 512 + kKeep + 128;  // 16-bit words
+template <bool MIXED, int W>
 __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_build(DevView v) {
     extern __shared__ __align__(16) unsigned char smem[];
     if (!v.flags->rebuild) return;
@@ -161,79 +224,87 @@ __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_build(DevVi
     CellGroup G = v.groups[blockIdx.x];
     int a0 = v.cell_start[G.cell], a1 = v.cell_start[G.cell + G.ncell];
     if (a0 == a1) return;
+    const int q0 = pair_first(a0, G.cell), q1 = pair_first(a1, G.cell + G.ncell);
     const SysDev &S = v.sys[G.sys];
     if (!S.nb_on) {
-        for (int i = a0 + threadIdx.x; i < a1; i += blockDim.x) v.ncount[i] = 0;
+        for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) v.ncount[q] = make_int2(0, 0);
         return;
     }
     int cap = v.hood_cap;
     float4 *s_q = reinterpret_cast<float4 *>(smem);  // .w: the original index's bits
-    uint16_t *s_buf = reinterpret_cast<uint16_t *>(s_q + cap);  // [W][2][256], 16-byte aligned
-    int *s_bnd = reinterpret_cast<int *>(s_buf + W * 512);
+    // per warp: a list's two chunks in the making (512 entries), the entries
+    // kept for its end (kKeep), the two atoms' exclusion partners (2 x 32)
+    uint16_t *s_buf = reinterpret_cast<uint16_t *>(s_q + cap);
+    int *s_bnd = reinterpret_cast<int *>(s_buf + W * kBuildWarpWords);
     HoodSpan *spans = reinterpret_cast<HoodSpan *>(s_bnd + 25 * (kRowCells + 1));
     int *s_n = reinterpret_cast<int *>(spans + kMaxSpans);
     __shared__ float4 s_dt[25 * kRowCells];
-    int c3f = v.cell3[a0];
     load_dtab(v, G.sys, s_dt);
-    int n = hood_setup(v, S, c3f, G.ncell, spans, s_n, s_bnd);
+    int n = hood_setup(v, S, v.cell3[a0], G.ncell, spans, s_n, s_bnd);
     int nsp = s_n[1];
+    // the group's own atoms are consecutive in the tile from here on
+    const int kbase = s_bnd[12 * (kRowCells + 1) + 2] - a0;
     // the spans, for the pair kernel's steps until the next rebuild
     {
         const int *src = reinterpret_cast<const int *>(spans);
         int *dst = v.gspan + (size_t)blockIdx.x * kGroupSpanWords;
         for (int e = threadIdx.x; e < min(nsp, kMaxSpans) * kSpanWords; e += blockDim.x) dst[e] = src[e];
-        if (threadIdx.x == 0) v.gspan_n[blockIdx.x] = make_int2(n, nsp);
+        if (threadIdx.x == 0) v.gspan_n[blockIdx.x] = make_int4(n, nsp, kbase, 0);
     }
     if (n > v.hood_cap || nsp > kMaxSpans) {
         if (threadIdx.x == 0) atomicOr(&v.flags->error, ERR_NLIST_OVERFLOW);
         return;
     }
-    if (v.mixed)
-        stage<true, true>(v, S, s_q, nullptr, spans, nsp, s_dt);
-    else
-        stage<true, false>(v, S, s_q, nullptr, spans, nsp, s_dt);
+    stage<true, MIXED>(v, S, s_q, nullptr, spans, nsp, s_dt);
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     float rl2 = S.rlist2f * 1.0001f + 1e-6f;
     const float margin = 0.01f;
     const float rlm = sqrtf(rl2) + margin;
     const float csx = (float)S.cs[0], csy = (float)S.cs[1], csz = (float)S.cs[2], icsz = 1.0f / csz;
-    int czf = (c3f >> 20) & 1023;
     int g = G.ncell;
-    for (int i = a0 + warp; i < a1; i += nw) {
-        float pi3[3];
-        i_in_group_frame(v, S, i, czf, pi3);
-        int oi = v.orig[i];
-        int e0 = v.excl_off[oi];
-        int ne = v.excl_off[oi + 1] - e0;
-        int my_ex = lane < ne ? v.excl_lst[e0 + lane] : -1;
-        int nfast = ne < 32 ? ne : 32;
-        // Index window [ex_lo, ex_lo + ex_win] of i itself and its exclusion
-        // partners (rows ascending): a candidate outside it needs no
-        // membership test.  i is left out by its index too, so every image
-        // of i is (the far one lies beyond the list radius anyway).
-        const int ex_lo = ne ? min(v.excl_lst[e0], oi) : oi;
-        const unsigned ex_win = (unsigned)((ne ? max(v.excl_lst[e0 + ne - 1], oi) : oi) - ex_lo);
-        int count = 0;
-        uint16_t *out = v.nl16 + (size_t)i * v.stride;
-        // lane r < 25: the tile range [kb, ke) of row r that i's sphere reaches
+    uint16_t *buf = s_buf + warp * kBuildWarpWords, *keep = buf + 512;
+    const unsigned q_addr = smem_addr(s_q), buf_addr = smem_addr(buf), keep_addr = smem_addr(keep),
+                   ex_addr = keep_addr + 2 * kKeep, lt = (1u << lane) - 1u;
+    const int cap_entries = pair_stride(v.stride);
+    for (int q = q0 + warp; q < q1; q += nw) {
+        const int2 ab = v.ipair[q];
+        if (ab.x < 0) continue;
+        BuildAtom A, B;
+        A.load(v, s_q[kbase + ab.x], ex_addr, lane);
+        B.load(v, s_q[kbase + (ab.y < 0 ? ab.x : ab.y)], ex_addr + 128, lane);
+        if (ab.y < 0) B.x = B.y = B.z = 1e15f;  // no second atom: beyond every list radius
+        __syncwarp();
+        int count = 0, kept = 0;
+        unsigned flagged = 0;  // chunks with an entry that is excluded from one of the two
+        uint16_t *out = pair_list(v, q);
+        // lane r < 25: the tile range [kb, ke) of row r that a sphere reaches
         int kb = 0, ke = 0;
         if (lane < 25) {
-            // distance from i to the row's cell column in x and y
-            float ox = (float)(lane / 5 - 2), oy = (float)(lane % 5 - 2);
-            float ddx = fmaxf(fmaxf(ox * csx - pi3[0], pi3[0] - (ox + 1.0f) * csx), 0.0f);
-            float ddy = fmaxf(fmaxf(oy * csy - pi3[1], pi3[1] - (oy + 1.0f) * csy), 0.0f);
-            float rem = rlm * rlm - (ddx * ddx + ddy * ddy);
-            if (rem >= 0.0f) {
-                float h = sqrtf(rem) + margin;
-                int zlo = max((int)floorf((pi3[2] - h) * icsz), -2);
-                int zhi = min((int)floorf((pi3[2] + h) * icsz), g + 1);
+            // z extent of the two spheres over the row: distance from each
+            // atom to the row's cell column in x and y
+            const float ox = (float)(lane / 5 - 2) * csx, oy = (float)(lane % 5 - 2) * csy;
+            float zl = 1e30f, zh = -1e30f;
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const float px = m ? B.x : A.x, py = m ? B.y : A.y, pz = m ? B.z : A.z;
+                const float ddx = fmaxf(fmaxf(ox - px, px - (ox + csx)), 0.0f);
+                const float ddy = fmaxf(fmaxf(oy - py, py - (oy + csy)), 0.0f);
+                const float rem = rlm * rlm - (ddx * ddx + ddy * ddy);
+                if (rem >= 0.0f) {
+                    const float h = sqrtf(rem) + margin;
+                    zl = fminf(zl, pz - h);
+                    zh = fmaxf(zh, pz + h);
+                }
+            }
+            if (zl <= zh) {
+                int zlo = max((int)floorf(zl * icsz), -2);
+                int zhi = min((int)floorf(zh * icsz), g + 1);
                 if (zlo <= zhi) {
                     const int *b = s_bnd + lane * (kRowCells + 1);
                     // the row is sorted by z (cells in z order, atoms in a
-                    // cell by z): narrow to the atoms with z in pz +- h.  The
+                    // cell by z): narrow to the atoms with z in [zl, zh].  The
                     // first such atom lies in cell zlo and the last in cell
                     // zhi, so each search covers one cell.
-                    const float zl = pi3[2] - h, zh = pi3[2] + h;
                     int l = b[zlo + 2], r = b[zlo + 3];
                     while (l < r) {
                         int mid = (l + r) >> 1;
@@ -256,60 +327,104 @@ __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_build(DevVi
                 }
             }
         }
-        // i's list is assembled per 256-entry chunk in two halves per warp
+        // The list is assembled per 256-entry chunk in two halves per warp
         // (entry p at p & 511), so an iteration that completes a chunk writes
         // on into the other half; a completed chunk is stored transposed as
-        // in memory (lane l's 16 bytes hold entries l + 32 q, q = 0..7)
-        uint16_t *buf = s_buf + warp * 512;
-        const unsigned lt = (1u << lane) - 1u;
+        // in memory (lane l's 16 bytes hold entries l + 32 q, q = 0..7).
+        // Every lane stores: a rejected candidate goes to count + 32 + lane,
+        // past the entries of this iteration -- a slot that a later entry
+        // overwrites or that lies beyond the list's count (never in the half
+        // being stored: at most 32 entries come per iteration).
+        auto append = [&](bool cand, int entry) {
+            const unsigned m = __ballot_sync(full, cand);
+            const int newc = count + __popc(m);
+            const int at = (cand ? count + __popc(m & lt) : count + 32 + lane) & 511;
+            sts16(buf_addr + 2 * at, entry);
+            if ((newc ^ count) >> 8) {
+                // chunk count >> 8 complete: one 16-byte store per lane
+                __syncwarp();
+                const int c = count >> 8;
+                if ((c + 1) * 256 <= cap_entries) store_chunk(out + c * 256, buf + (c & 1) * 256, lane);
+                __syncwarp();
+            }
+            count = newc;
+        };
         unsigned rows = __ballot_sync(full, ke > kb);
         while (rows) {
             int r = __ffs(rows) - 1;
             rows &= rows - 1;
             const int rb = __shfl_sync(full, kb, r), re = __shfl_sync(full, ke, r);
-            for (int k0 = rb; k0 < re; k0 += 32) {
+            for (int k = rb + lane; k - lane < re; k += 32) {
                 // k past the row's end reads a later row or the chunk
                 // buffers behind the tile, inside the block's shared
                 // memory; such a lane is no candidate
-                const int k = k0 + lane;
-                const float4 q = s_q[k];
-                const float dx = pi3[0] - q.x, dy = pi3[1] - q.y, dz = pi3[2] - q.z;
-                bool cand = (k < re) & (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < rl2);
-                const int oj = __float_as_int(q.w);
-                if (__any_sync(full, cand && (unsigned)(oj - ex_lo) <= ex_win)) {
-                    bool ex = oj == oi;
-                    for (int e = 0; e < nfast; ++e) ex |= (__shfl_sync(full, my_ex, e) == oj);
-                    if (ne > 32 && cand)
-                        for (int e = 32; e < ne; ++e) ex |= (v.excl_lst[e0 + e] == oj);
-                    cand = cand && !ex;
+                const float4 c = lds128(q_addr + 16 * k);
+                const bool in_row = k < re;
+                bool inA = in_row & (A.r2(c) < rl2), inB = in_row & (B.r2(c) < rl2);
+                const int oj = __float_as_int(c.w);
+                int entry = k << kEntryShift;
+                bool cand = inA | inB;
+                if (__any_sync(full, cand && ((unsigned)(oj - A.lo) <= A.win || (unsigned)(oj - B.lo) <= B.win))) {
+                    const bool exA = A.excluded(v, oj), exB = B.excluded(v, oj);
+                    inA &= !exA;
+                    inB &= !exB;
+                    cand = inA | inB;
+                    entry |= (exA ? 1 : 0) | (exB ? 2 : 0);
+                    // excluded from one of the two: kept for the list's end
+                    // while there is room
+                    const unsigned m = __ballot_sync(full, cand && (exA || exB));
+                    if (kept + __popc(m) <= kKeep) {
+                        if ((m >> lane) & 1) sts16(keep_addr + 2 * (kept + __popc(m & lt)), entry);
+                        kept += __popc(m);
+                        cand = cand && !((m >> lane) & 1);
+                    } else {
+                        // (an iteration's entries lie in the chunks of its
+                        // first and its last possible place)
+                        flagged |= 1u << (count >> 8) | 1u << min((count + 31) >> 8, 31);
+                    }
                 }
-                const unsigned m = __ballot_sync(full, cand);
-                const int newc = count + __popc(m);
-                // every lane stores: a rejected candidate goes to count + 32 +
-                // lane, past the entries of this iteration -- a slot that a
-                // later entry overwrites or that lies beyond the list's count
-                // (never in the half being stored: at most 32 entries come
-                // per iteration)
-                buf[(cand ? count + __popc(m & lt) : count + 32 + lane) & 511] = (uint16_t)(k << kEntryShift);
-                if ((newc ^ count) >> 8) {
-                    // chunk count >> 8 complete: one 16-byte store per lane
-                    __syncwarp();
-                    const int c = count >> 8;
-                    if ((c + 1) * 256 <= v.stride) store_chunk(out + c * 256, buf + (c & 1) * 256, lane);
-                    __syncwarp();
-                }
-                count = newc;
+                // The FP64 kernel and the pair set take an entry's atom at its
+                // nearest image; in a box of few cells the tile holds two
+                // images of an atom, one for either atom of the pair, so
+                // there an entry counts only for the atoms it is near
+                // (marked in FP64 only: the mixed kernel takes the tile's image)
+                if (!MIXED) entry |= (inA ? 0 : 1) | (inB ? 0 : 2);
+                append(cand, entry);
             }
         }
         __syncwarp();
-        {
-            const int c = count >> 8;
-            if ((count & 255) && c * 256 < v.stride) store_chunk(out + c * 256, buf + (c & 1) * 256, lane);
+        for (int t0 = 0; t0 < kept; t0 += 32) {
+            flagged |= 1u << (count >> 8) | 1u << min((count + 31) >> 8, 31);
+            append(t0 + lane < kept, keep[min(t0 + lane, kKeep - 1)]);
         }
         __syncwarp();
+        if (((count + lane) ^ count) < 32 && (count & 31)) sts16(buf_addr + 2 * ((count + lane) & 511), cap << kEntryShift);
+        __syncwarp();
+        {
+            const int c = count >> 8;
+            if ((count & 255) && (c + 1) * 256 <= cap_entries) store_chunk(out + c * 256, buf + (c & 1) * 256, lane);
+        }
+        __syncwarp();
+        bool over = false;
+        if (count > v.stride) {
+            // The capacity is an atom's: its own entries, whatever the
+            // union's count.  Counted apart, as it is hardly ever asked.
+            int nA = 0, nB = 0;
+            for (unsigned left = __ballot_sync(full, ke > kb); left; left &= left - 1) {
+                const int r = __ffs(left) - 1;
+                const int rb = __shfl_sync(full, kb, r), re = __shfl_sync(full, ke, r);
+                for (int k = rb + lane; k < re; k += 32) {
+                    const float4 c = s_q[k];
+                    const int oj = __float_as_int(c.w);
+                    nA += A.r2(c) < rl2 && !A.excluded(v, oj);
+                    nB += B.r2(c) < rl2 && !B.excluded(v, oj);
+                }
+            }
+            over = max(__reduce_add_sync(full, nA), __reduce_add_sync(full, nB)) > v.stride;
+        }
         if (lane == 0) {
-            v.ncount[i] = count < v.stride ? count : v.stride;
-            if (count > v.stride) atomicOr(&v.flags->error, ERR_NLIST_OVERFLOW);
+            v.ncount[q] = make_int2(over ? 0 : count, (int)flagged);
+            if (over) atomicOr(&v.flags->error, ERR_NLIST_OVERFLOW);
         }
     }
 }
@@ -317,8 +432,7 @@ __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_build(DevVi
 // ------------------------------------------------------------------ pairs
 
 struct PairPrm {
-    float ex2c, a04, k2a, sw, cut;  // SysDev::ex2c, a04, k2a
-    int use_sw;
+    float ex2c, a04, k2a, sw, inv_w;  // SysDev::ex2c, a04, k2a; the switching distance, 1 / its width
 };
 
 __device__ __forceinline__ float fast_ex2(float x) {
@@ -326,53 +440,6 @@ __device__ __forceinline__ float fast_ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-
-// FP32 force (and energy) of one list entry, accumulated into the lane's
-// partial sums when `in` (inside the cutoff), NonbondedForce.cpp:559-581 in
-// single precision.  Evaluated without branches: an entry outside the cutoff
-// (r^2 up to 1e30 for padding) gives finite values that the select drops, so
-// two entries per lane run as independent instruction streams.
-template <bool ENERGY, bool SW>
-__device__ __forceinline__ void pair_mixed(bool in, float dx, float dy, float dz, float r2, float qq, float sg,
-                                           float eps, const PairPrm &P, float &fx, float &fy, float &fz,
-                                           float &ec, float &ev) {
-    float rinv = fast_rsqrt(r2);
-    float rinv2 = rinv * rinv;
-    float r = r2 * rinv;
-    // exp(-(alpha r)^2) straight from r^2; erfc(alpha r) = exp(-(alpha r)^2) g(t),
-    // t = 1 / (1 + 0.4 alpha r); 2 alpha r / sqrt(pi) as k2a * r
-    float ex = fast_ex2(r2 * P.ex2c);
-    float erfcv = ex * erfcx_fit(fast_rcp(fmaf(P.a04, r, 1.0f)));
-    float qr = qq * rinv;
-    float dEdR = qr * rinv2 * fmaf(P.k2a * r, ex, erfcv);
-    float s2 = sg * sg * rinv2;
-    float s6 = s2 * s2 * s2;
-    float evdw = eps * (s6 - 1.0f) * s6;
-    float sw = 1.0f;
-    if (SW && P.use_sw && r > P.sw) {
-        float w = P.cut - P.sw;
-        float t = (r - P.sw) / w;
-        sw = 1.0f + t * t * t * (-10.0f + t * (15.0f - t * 6.0f));
-        float dsw = t * t * (-30.0f + t * (60.0f - t * 30.0f)) / w;
-        dEdR -= evdw * dsw * rinv;
-    }
-    float lj = eps * (12.0f * s6 - 6.0f) * s6;
-    if (SW) lj *= sw;
-    dEdR = fmaf(lj, rinv2, dEdR);
-    dEdR = in ? dEdR : 0.0f;
-    fx = fmaf(dx, dEdR, fx);
-    fy = fmaf(dy, dEdR, fy);
-    fz = fmaf(dz, dEdR, fz);
-    if (ENERGY) {
-        ec += in ? qr * erfcv : 0.0f;
-        ev += in ? (SW ? sw * evdw : evdw) : 0.0f;
-    }
-}
-
-// Per-system constants of pair_mixed2, each in both halves of a float2.
-struct PairPrm2 {
-    float2 ex2c, a04, k2a, one, twelve, msix, mone;
-};
 
 __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 
@@ -387,49 +454,124 @@ __device__ __forceinline__ float2 erfcx_fit2(float2 t) {
     return g;
 }
 
-// pair_mixed for a lane's two entries at once (no switching function): the
-// same chain of operations per entry in the two halves of packed FP32x2
-// arithmetic, one instruction for both entries (the reciprocal square root,
-// exponential and reciprocal stay scalar); about a sixth fewer instructions
-// per entry.  The displacements come as j - i, so the force sums (fxy = x,
-// y; fz) are negated sums; the caller flips their sign.
-template <bool ENERGY>
-__device__ __forceinline__ void pair_mixed2(bool in0, bool in1, float2 dxy0, float dz0, float2 dxy1, float dz1,
-                                            float2 r2, float2 qq, float2 sg, float2 eps, const PairPrm2 &P,
-                                            float2 &fxy, float &fz, float2 &ecv) {
-    float2 rinv = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
-    float2 rinv2 = __fmul2_rn(rinv, rinv);
-    float2 r = __fmul2_rn(r2, rinv);
-    float2 ea = __fmul2_rn(r2, P.ex2c);
-    float2 ex = make_float2(fast_ex2(ea.x), fast_ex2(ea.y));
-    float2 tt = __ffma2_rn(P.a04, r, P.one);
-    float2 erfcv = __fmul2_rn(ex, erfcx_fit2(make_float2(fast_rcp(tt.x), fast_rcp(tt.y))));
-    float2 qr = __fmul2_rn(qq, rinv);
-    float2 dEdR = __fmul2_rn(__fmul2_rn(qr, rinv2), __ffma2_rn(__fmul2_rn(P.k2a, r), ex, erfcv));
-    float2 s2 = __fmul2_rn(__fmul2_rn(sg, sg), rinv2);
-    float2 s6 = __fmul2_rn(__fmul2_rn(s2, s2), s2);
+// The two atoms of a pair against one list entry: FP32 force (and energy) of
+// both, NonbondedForce.cpp:559-581 in single precision, in the two halves of
+// packed FP32x2 operations (one instruction for both; the reciprocal square
+// root, exponential and reciprocal are scalar), added to the lane's sums
+// where `in`.  Without branches: an entry outside the cutoff gives finite
+// values that a select drops (with energies: selects on the charge product
+// and epsilon, which every term has as a factor; four selects for six).
+// exp(-(alpha r)^2) comes straight from r^2; erfc(alpha r) =
+// exp(-(alpha r)^2) g(t), t = 1 / (1 + 0.4 alpha r).
+struct PairSums {
+    float2 fx, fy, fz, ec, ev;  // .x: the first atom, .y: the second
+};
 
-    float2 lj = __fmul2_rn(__fmul2_rn(eps, __ffma2_rn(P.twelve, s6, P.msix)), s6);
-    dEdR = __ffma2_rn(lj, rinv2, dEdR);
-    const float d0 = in0 ? dEdR.x : 0.0f, d1 = in1 ? dEdR.y : 0.0f;
-    fxy = __ffma2_rn(dxy0, dup2(d0), fxy);
-    fz = fmaf(dz0, d0, fz);
-    fxy = __ffma2_rn(dxy1, dup2(d1), fxy);
-    fz = fmaf(dz1, d1, fz);
+template <bool ENERGY, bool SW>
+__device__ __forceinline__ void pair_mixed2(bool in0, bool in1, float2 dx, float2 dy, float2 dz, float2 r2, float2 qq,
+                                            float2 sg, float2 eps, const PairPrm &P, PairSums &F) {
     if (ENERGY) {
-        // (Coulomb, LJ) as one packed sum, entry 0 then entry 1 (entries
-        // outside the cutoff add zero)
-        const float2 e = __fmul2_rn(qr, erfcv);
-        const float2 l = __fmul2_rn(__fmul2_rn(eps, __fadd2_rn(s6, P.mone)), s6);
-        ecv = __fadd2_rn(ecv, make_float2(in0 ? e.x : 0.0f, in0 ? l.x : 0.0f));
-        ecv = __fadd2_rn(ecv, make_float2(in1 ? e.y : 0.0f, in1 ? l.y : 0.0f));
+        qq = make_float2(in0 ? qq.x : 0.0f, in1 ? qq.y : 0.0f);
+        eps = make_float2(in0 ? eps.x : 0.0f, in1 ? eps.y : 0.0f);
+    }
+    const float2 rinv = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
+    const float2 rinv2 = __fmul2_rn(rinv, rinv);
+    const float2 r = __fmul2_rn(r2, rinv);
+    const float2 ea = __fmul2_rn(r2, dup2(P.ex2c));
+    const float2 ex = make_float2(fast_ex2(ea.x), fast_ex2(ea.y));
+    const float2 tt = __ffma2_rn(dup2(P.a04), r, dup2(1.0f));
+    const float2 erfcv = __fmul2_rn(ex, erfcx_fit2(make_float2(fast_rcp(tt.x), fast_rcp(tt.y))));
+    const float2 qr = __fmul2_rn(qq, rinv);
+    float2 dEdR = __fmul2_rn(__fmul2_rn(qr, rinv2), __ffma2_rn(__fmul2_rn(dup2(P.k2a), r), ex, erfcv));
+    if (ENERGY) F.ec = __ffma2_rn(qr, erfcv, F.ec);
+    const float2 s2 = __fmul2_rn(__fmul2_rn(sg, sg), rinv2);
+    const float2 s6 = __fmul2_rn(__fmul2_rn(s2, s2), s2);
+    const float2 es6 = __fmul2_rn(eps, s6);
+    float2 lj = __fmul2_rn(es6, __ffma2_rn(dup2(12.0f), s6, dup2(-6.0f)));
+    if (SW) {
+        // t = 0 before the switching distance (and where the system has no
+        // switch): the factor is 1 and its derivative 0; at most 1, so that an
+        // entry beyond every cutoff stays finite
+        const float2 u = __ffma2_rn(r, dup2(P.inv_w), dup2(-P.sw * P.inv_w));
+        const float2 t = make_float2(__saturatef(u.x), __saturatef(u.y));
+        const float2 t2 = __fmul2_rn(t, t);
+        const float2 sw = __ffma2_rn(__fmul2_rn(t2, t), __ffma2_rn(t, __ffma2_rn(t, dup2(-6.0f), dup2(15.0f)), dup2(-10.0f)),
+                                     dup2(1.0f));
+        const float2 mdsw = __fmul2_rn(__fmul2_rn(t2, dup2(P.inv_w)),
+                                       __ffma2_rn(t, __ffma2_rn(t, dup2(30.0f), dup2(-60.0f)), dup2(30.0f)));
+        const float2 l = __ffma2_rn(es6, s6, make_float2(-es6.x, -es6.y));
+        lj = __ffma2_rn(sw, lj, __fmul2_rn(__fmul2_rn(l, mdsw), r));
+        if (ENERGY) F.ev = __ffma2_rn(l, sw, F.ev);
+    } else if (ENERGY) {
+        F.ev = __fadd2_rn(F.ev, __ffma2_rn(es6, s6, make_float2(-es6.x, -es6.y)));
+    }
+    dEdR = __ffma2_rn(lj, rinv2, dEdR);
+    if (!ENERGY) dEdR = make_float2(in0 ? dEdR.x : 0.0f, in1 ? dEdR.y : 0.0f);
+    F.fx = __ffma2_rn(dx, dEdR, F.fx);
+    F.fy = __ffma2_rn(dy, dEdR, F.fy);
+    F.fz = __ffma2_rn(dz, dEdR, F.fz);
+}
+
+// The entries of one chunk (c0) of pair q's list whose FP32 r^2 is within
+// 1e-5 of the cutoff's, which the walk left out: decided in FP64 exactly as
+// the reference, and added where they are within it.  One chunk in a hundred
+// comes here.  The energies' kernel calls it when the pair is done, with its
+// own atomics, so that its registers are not added to the walk's (179 -> 157
+// us at 94,100 atoms).
+template <bool ENERGY, bool SW>
+__device__ __forceinline__ void near_cutoff(const DevView &v, const SysDev &S, const HoodSpan *spans, int nsp, int kbase,
+                                            int q, int c0, unsigned q_addr, unsigned lj_addr) {
+    const int lane = threadIdx.x & 31;
+    const int2 ab = v.ipair[q];
+    const int cnt = min(v.ncount[q].x, c0 + 256);
+    const uint16_t *list = pair_list(v, q);
+    const float inv_w = SW && S.use_switch ? 1.0f / (S.cutofff - S.sw_distf) : 0.0f;
+    const PairPrm P{S.ex2c, S.a04, S.k2a, inv_w != 0.0f ? S.sw_distf : 0.0f, inv_w};
+    for (int k = c0 + lane; k < cnt; k += 32) {
+        const unsigned w = list[list_pos(k)], e = w & 0xfff8u;
+        const float4 p = lds128(q_addr + 2 * e);
+        const float2 l = lds64(lj_addr + e);
+        for (int m = 0; m < 2; ++m) {
+            const int i = m ? ab.y : ab.x;
+            if (i < 0 || ((w >> m) & 1)) continue;
+            const float4 pi = lds128(q_addr + 16 * (kbase + i));
+            const float dx = pi.x - p.x, dy = pi.y - p.y, dz = pi.z - p.z;
+            const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+            if (!(r2 >= S.cut2f_lo && r2 < S.cut2f_hi)) continue;
+            if (!(exact_r2(v, S, i, hood_slot(spans, nsp, (int)(e >> kEntryShift))) < S.cut2)) continue;
+            const float2 li = lds64(lj_addr + 8 * (kbase + i));
+            PairSums F;
+            F.fx = F.fy = F.fz = F.ec = F.ev = make_float2(0.f, 0.f);
+            pair_mixed2<ENERGY, SW>(true, false, make_float2(dx, 0.f), make_float2(dy, 0.f), make_float2(dz, 0.f),
+                                    make_float2(r2, r2), make_float2(pi.w * p.w, 0.f), make_float2(li.x + l.x, 0.f),
+                                    make_float2(li.y * l.y, 0.f), P, F);
+            acc_add(static_cast<long long *>(v.fx) + i, F.fx.x);
+            acc_add(static_cast<long long *>(v.fy) + i, F.fy.x);
+            acc_add(static_cast<long long *>(v.fz) + i, F.fz.x);
+            if (ENERGY) {
+                long long *E = v.E + (size_t)v.sys_of[i] * E_SLOTS;
+                atomicAdd(reinterpret_cast<unsigned long long *>(E + E_COUL),
+                          static_cast<unsigned long long>(energy_fixed(0.5f * F.ec.x)));
+                atomicAdd(reinterpret_cast<unsigned long long *>(E + E_VDW),
+                          static_cast<unsigned long long>(energy_fixed(0.5f * F.ev.x)));
+            }
+        }
     }
 }
 
-// Mixed precision: each lane keeps two list entries in flight; j comes from
-// the staged tile.  SW: some system of the batch uses the switching function.
+// Mixed precision: one warp per pair of atoms walks the pair's list; j comes
+// from the staged tile, once for both.
+//
+// Bound by instruction issue and the FP32 pipe (a packed operation takes the
+// pipe for two).  An entry costs one load of j, one decoding and one set of
+// packed operations for two interactions, 12% of which the other atom's
+// share of the list adds: 145 -> 132 us at 94,100 atoms against a list per
+// atom, 189 -> 141 us with the switching function at 74,400, 101 -> 88 M warp
+// instructions.  Of its walk 57% of the cycles issue; the rest is the staging
+// before it and a block's last pairs.
+// SW: some system of the batch uses the switching function.
 template <bool ENERGY, bool SW, int W>
-__global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_pairs_mixed(DevView v) {
+__global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_pairs_mixed(const __grid_constant__ DevView v) {
     extern __shared__ __align__(16) unsigned char smem[];
     const unsigned full = 0xffffffffu;
     CellGroup G = v.groups[blockIdx.x];
@@ -437,146 +579,169 @@ __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_pairs_mixed
     if (a0 == a1) return;
     const SysDev &S = v.sys[G.sys];
     if (!S.nb_on) return;
-    int cap = v.hood_cap;
+    const int cap = v.hood_cap;
     // tile: LJ pairs first (a list entry is the byte offset of its atom's
     // pair), then positions at twice that offset past them (cap is a
     // multiple of 32, so the positions stay 16-byte aligned)
     float2 *s_lj = reinterpret_cast<float2 *>(smem);
-    float4 *s_q = reinterpret_cast<float4 *>(s_lj + cap);
-    HoodSpan *spans = reinterpret_cast<HoodSpan *>(s_q + cap);
-    const unsigned char *q_base = reinterpret_cast<const unsigned char *>(s_q);
+    float4 *s_q = reinterpret_cast<float4 *>(s_lj + cap + kTileSpare);
+    HoodSpan *spans = reinterpret_cast<HoodSpan *>(s_q + cap + kTileSpare);
     __shared__ float4 s_dt[25 * kRowCells];
-    __shared__ int2 s_nn;
-    int c3f = v.cell3[a0];
+    __shared__ int4 s_nn;
     // the neighbourhood's spans as the list build enumerated them (the
     // cells have not changed since), and the displacement table
     {
         const int *src = v.gspan + (size_t)blockIdx.x * kGroupSpanWords;
         int *dst = reinterpret_cast<int *>(spans);
         for (int e = threadIdx.x; e < kGroupSpanWords; e += blockDim.x) dst[e] = src[e];
-        if (threadIdx.x == 0) s_nn = v.gspan_n[blockIdx.x];
+        if (threadIdx.x == 0) {
+            s_nn = v.gspan_n[blockIdx.x];
+            // the spare place: an atom beyond every cutoff, without charge
+            // (the next: the second atom of a pair of one, as far the other way)
+            s_q[cap] = make_float4(1e15f, 1e15f, 1e15f, 0.f);
+            s_q[cap + 1] = make_float4(-1e15f, -1e15f, -1e15f, 0.f);
+            s_lj[cap] = s_lj[cap + 1] = make_float2(0.f, 0.f);
+        }
         const float4 *dt = v.dtab + G.sys * kDtabStride;
         for (int e = threadIdx.x; e < 25 * kRowCells; e += blockDim.x) s_dt[e] = __ldg(dt + e);
     }
     __syncthreads();
-    const int n = s_nn.x, nsp = s_nn.y;
+    const int n = s_nn.x, nsp = s_nn.y, kbase = s_nn.z;
     if (n > v.hood_cap || nsp > kMaxSpans) {
         if (threadIdx.x == 0) atomicOr(&v.flags->error, ERR_NLIST_OVERFLOW);
         return;
     }
+    // the warp's first pair, its counts and the first chunk of its list (whose
+    // place always exists: the load need not wait for the count) come in
+    // beside the staging, each later one's beside the sums before it
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int q1 = pair_first(a1, G.cell + G.ncell);
+    int2 ab, nc;
+    uint4 cur;
+    auto fetch = [&](int q) {
+        if (q >= q1) return;
+        ab = v.ipair[q];
+        nc = v.ncount[q];
+        cur = __ldg(reinterpret_cast<const uint4 *>(pair_list(v, q)) + lane);
+    };
+    int q = pair_first(a0, G.cell) + warp;
+    fetch(q);
     stage<false, true>(v, S, s_q, s_lj, spans, nsp, s_dt);
-    int czf = (c3f >> 20) & 1023;
-    const float lo = S.cut2f_lo, hi = S.cut2f_hi;
-    const PairPrm P{S.ex2c, S.a04, S.k2a, S.sw_distf, S.cutofff, S.use_switch};
-    const PairPrm2 P2{dup2(S.ex2c), dup2(S.a04), dup2(S.k2a), dup2(1.0f), dup2(12.0f), dup2(-6.0f), dup2(-1.0f)};
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    float ec = 0.f, ev = 0.f;
-    float2 ecv = make_float2(0.f, 0.f);  // pair_mixed2's (Coulomb, LJ) sums
-    for (int i = a0 + warp; i < a1; i += nw) {
-        float pi3[3];
-        i_in_group_frame(v, S, i, czf, pi3);
-        const float qi = v.pf[i].w;
-        const float2 li = v.ljf[i];
-        const int cnt = v.ncount[i];
-        const uint4 *lst4 = reinterpret_cast<const uint4 *>(v.nl16 + (size_t)i * v.stride) + lane;
-        float fx = 0.f, fy = 0.f, fz = 0.f;
-        // without the switching function: negated x, y sums as a pair (pair_mixed2)
-        float2 fxy = make_float2(0.f, 0.f);
-        const float2 nxy = make_float2(-pi3[0], -pi3[1]);
-        const float nz = -pi3[2];
-        // the first chunk's slot always exists: its load need not wait for the count
-        uint4 cur = __ldg(lst4);
+    const unsigned q_addr = smem_addr(s_q), lj_addr = smem_addr(s_lj);
+    const float lo = S.cut2f_lo, cut2 = S.cut2f;
+    const float inv_w = SW && S.use_switch ? 1.0f / (S.cutofff - S.sw_distf) : 0.0f;
+    const PairPrm P{S.ex2c, S.a04, S.k2a, inv_w != 0.0f ? S.sw_distf : 0.0f, inv_w};
+    PairSums F;
+    F.ec = F.ev = make_float2(0.f, 0.f);
+    while (q < q1) {
+        const uint4 *lst4 = reinterpret_cast<const uint4 *>(pair_list(v, q)) + lane;
+        q += W;
+        if (ab.x < 0) {
+            fetch(q);
+            continue;
+        }
+        const int cnt = nc.x;
+        const int ka = kbase + ab.x, kb = ab.y < 0 ? cap + 1 : kbase + ab.y;
+        const float4 pa = s_q[ka];
+        const float4 pb = s_q[kb];
+        const float2 la = s_lj[ka], lb = s_lj[kb];
+        F.fx = F.fy = F.fz = make_float2(0.f, 0.f);
+        unsigned near = 0;  // chunks with an entry at the cutoff (energies)
         for (int c0 = 0; c0 < cnt; c0 += 256) {
+            float edge = 1e30f;  // the least distance of an FP32 r^2 from the cutoff's
             // this lane's entries c0 + lane + 32u, u = 0..7, and the next chunk in flight
             uint4 nxt = c0 + 256 < cnt ? __ldg(lst4 + (c0 + 256) / 8) : make_uint4(0, 0, 0, 0);
-            uint32_t wds[4] = {cur.x, cur.y, cur.z, cur.w};
-            // bit u: entry u's FP32 r^2 lies within 1e-5 of the cutoff, so
-            // the FP32 test (which left it out) is re-done in FP64 below
-            unsigned amb = 0;
-            // FULL: all 256 entries of the chunk are valid (every chunk but
-            // the last), so the per-entry range checks compile away
-            auto walk = [&](auto full_chunk) {
-                constexpr bool FULL = decltype(full_chunk)::value;
-#pragma unroll
-                for (int u = 0; u < 8; u += 2) {
-                    if (!FULL && c0 + 32 * u >= cnt) break;  // rest of the last chunk is empty (warp-uniform)
-                    int k0 = c0 + lane + 32 * u;
-                    bool v0 = FULL || k0 < cnt, v1 = FULL || k0 + 32 < cnt;
-                    const unsigned e0 = v0 ? (wds[u >> 1] & 0xffffu) : 0u;
-                    const unsigned e1 = v1 ? (wds[u >> 1] >> 16) : 0u;
-                    const float4 p0 = *reinterpret_cast<const float4 *>(q_base + 2 * e0);
-                    const float4 p1 = *reinterpret_cast<const float4 *>(q_base + 2 * e1);
-                    const float2 l0 = *reinterpret_cast<const float2 *>(smem + e0);
-                    const float2 l1 = *reinterpret_cast<const float2 *>(smem + e1);
-                    // j - i: x and y as one pair per entry
-                    const float2 dxy0 = __fadd2_rn(make_float2(p0.x, p0.y), nxy);
-                    const float2 dxy1 = __fadd2_rn(make_float2(p1.x, p1.y), nxy);
-                    const float dz0 = p0.z + nz, dz1 = p1.z + nz;
-                    float r20 = v0 ? fmaf(dz0, dz0, fmaf(dxy0.y, dxy0.y, dxy0.x * dxy0.x)) : 1e30f;
-                    float r21 = v1 ? fmaf(dz1, dz1, fmaf(dxy1.y, dxy1.y, dxy1.x * dxy1.x)) : 1e30f;
-                    const bool in0 = r20 < lo, in1 = r21 < lo;
-                    amb |= ((!in0 && r20 < hi) ? 1u : 0u) << u;
-                    amb |= ((!in1 && r21 < hi) ? 1u : 0u) << (u + 1);
-                    if (SW) {
-                        pair_mixed<ENERGY, SW>(in0, -dxy0.x, -dxy0.y, -dz0, r20, qi * p0.w, li.x + l0.x,
-                                               li.y * l0.y, P, fx, fy, fz, ec, ev);
-                        pair_mixed<ENERGY, SW>(in1, -dxy1.x, -dxy1.y, -dz1, r21, qi * p1.w, li.x + l1.x,
-                                               li.y * l1.y, P, fx, fy, fz, ec, ev);
-                    } else {
-                        pair_mixed2<ENERGY>(in0, in1, dxy0, dz0, dxy1, dz1, make_float2(r20, r21),
-                                            make_float2(qi * p0.w, qi * p1.w), make_float2(li.x + l0.x, li.x + l1.x),
-                                            make_float2(li.y * l0.y, li.y * l1.y), P2, fxy, fz, ecv);
-                    }
+            // FLAGS: the entry may be excluded from one of the two atoms
+            auto entry = [&](unsigned w, auto flags) {
+                constexpr bool FLAGS = decltype(flags)::value;
+                const unsigned e = FLAGS ? w & 0xfff8u : w;
+                const float4 p = lds128(q_addr + 2 * e);
+                const float2 l = lds64(lj_addr + e);
+                const float2 dx = make_float2(pa.x - p.x, pb.x - p.x);
+                const float2 dy = make_float2(pa.y - p.y, pb.y - p.y);
+                const float2 dz = make_float2(pa.z - p.z, pb.z - p.z);
+                float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+                if (FLAGS) {
+                    if (w & 1) r2.x = 1e30f;
+                    if (w & 2) r2.y = 1e30f;
                 }
+                const float2 off = __fadd2_rn(r2, dup2(-cut2));
+                edge = fminf(edge, fminf(fabsf(off.x), fabsf(off.y)));
+                pair_mixed2<ENERGY, SW>(r2.x < lo, r2.y < lo, dx, dy, dz, r2, make_float2(pa.w * p.w, pb.w * p.w),
+                                        make_float2(la.x + l.x, lb.x + l.x), make_float2(la.y * l.y, lb.y * l.y), P,
+                                        F);
             };
-            if (c0 + 256 <= cnt)
-                walk(std::true_type{});
-            else
-                walk(std::false_type{});
-            if (__any_sync(full, amb != 0)) {
-                // near the cutoff: decide in FP64 exactly as the reference;
-                // an entry within the cutoff is evaluated here (the walk
-                // dropped it)
-                for (int u = 0; u < 8; ++u) {
-                    if (!((amb >> u) & 1u)) continue;
-                    const unsigned e = (wds[u >> 1] >> (16 * (u & 1))) & 0xffffu;
-                    if (!(exact_r2(v, S, i, hood_slot(spans, nsp, (int)(e >> kEntryShift))) < S.cut2)) continue;
-                    const float4 pj = *reinterpret_cast<const float4 *>(q_base + 2 * e);
-                    const float2 lj = *reinterpret_cast<const float2 *>(smem + e);
-                    // j - i, the walk's convention (the sums are negated at the end)
-                    const float dx = pj.x - pi3[0], dy = pj.y - pi3[1], dz = pj.z - pi3[2];
-                    const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                    if (SW)
-                        pair_mixed<ENERGY, SW>(true, -dx, -dy, -dz, r2, qi * pj.w, li.x + lj.x, li.y * lj.y, P, fx,
-                                               fy, fz, ec, ev);
-                    else
-                        pair_mixed<ENERGY, SW>(true, dx, dy, dz, r2, qi * pj.w, li.x + lj.x, li.y * lj.y, P, fxy.x,
-                                               fxy.y, fz, ec, ev);
+            if (c0 + 256 <= cnt && !((nc.y >> (c0 >> 8)) & 1)) {
+                const uint32_t wds[4] = {cur.x, cur.y, cur.z, cur.w};
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    entry((u & 1) ? wds[u >> 1] >> 16 : wds[u >> 1] & 0xffffu, std::false_type{});
+            } else {
+                uint4 w = cur;
+                for (int u0 = c0; u0 < min(cnt, c0 + 256); u0 += 32) {
+                    entry(w.x & 0xffffu, std::true_type{});
+                    w.x = __funnelshift_r(w.x, w.y, 16);
+                    w.y = __funnelshift_r(w.y, w.z, 16);
+                    w.z = __funnelshift_r(w.z, w.w, 16);
+                    w.w >>= 16;
+                }
+            }
+            if (__any_sync(full, edge < cut2 * 1.1e-5f)) {
+                if constexpr (ENERGY) {
+                    near |= 1u << (c0 >> 8);
+                } else {
+                    // at once, into the walk's sums
+                    uint4 ws = cur;
+                    for (int u0 = c0; u0 < min(cnt, c0 + 256); u0 += 32) {
+                        const unsigned w = ws.x & 0xffffu, e = w & 0xfff8u;
+                        ws.x = __funnelshift_r(ws.x, ws.y, 16);
+                        ws.y = __funnelshift_r(ws.y, ws.z, 16);
+                        ws.z = __funnelshift_r(ws.z, ws.w, 16);
+                        ws.w >>= 16;
+                        const float4 p = lds128(q_addr + 2 * e);
+                        const float2 l = lds64(lj_addr + e);
+                        const float2 dx = make_float2(pa.x - p.x, pb.x - p.x);
+                        const float2 dy = make_float2(pa.y - p.y, pb.y - p.y);
+                        const float2 dz = make_float2(pa.z - p.z, pb.z - p.z);
+                        const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+                        bool in0 = !(w & 1) && r2.x >= lo && r2.x < S.cut2f_hi;
+                        bool in1 = !(w & 2) && r2.y >= lo && r2.y < S.cut2f_hi;
+                        if (!(in0 || in1)) continue;
+                        const int j = hood_slot(spans, nsp, (int)(e >> kEntryShift));
+                        in0 = in0 && exact_r2(v, S, ab.x, j) < S.cut2;
+                        in1 = in1 && exact_r2(v, S, ab.y, j) < S.cut2;
+                        pair_mixed2<ENERGY, SW>(in0, in1, dx, dy, dz, r2, make_float2(pa.w * p.w, pb.w * p.w),
+                                                make_float2(la.x + l.x, lb.x + l.x),
+                                                make_float2(la.y * l.y, lb.y * l.y), P, F);
+                    }
                 }
             }
             cur = nxt;
         }
-        if (!SW) {
-            fx = -fxy.x;
-            fy = -fxy.y;
-            fz = -fz;
-        }
-        fx = warp_sum(fx);
-        fy = warp_sum(fy);
-        fz = warp_sum(fz);
-        if (lane == 0) {
-            acc_add(static_cast<long long *>(v.fx) + i, fx);
-            acc_add(static_cast<long long *>(v.fy) + i, fy);
-            acc_add(static_cast<long long *>(v.fz) + i, fz);
-        }
+        const int2 at = ab;
+        fetch(q);
+        // six sums over 32 lanes in eight steps: lanes take a share of the
+        // sums at each of the first three (bit 4 of the lane: the atom; then
+        // bit 3 x or y; bit 2 set: z)
+        const bool up16 = lane & 16, up8 = lane & 8, up4 = lane & 4;
+        float sx = (up16 ? F.fx.y : F.fx.x) + __shfl_xor_sync(full, up16 ? F.fx.x : F.fx.y, 16);
+        float sy = (up16 ? F.fy.y : F.fy.x) + __shfl_xor_sync(full, up16 ? F.fy.x : F.fy.y, 16);
+        float sz = (up16 ? F.fz.y : F.fz.x) + __shfl_xor_sync(full, up16 ? F.fz.x : F.fz.y, 16);
+        sx = (up8 ? sy : sx) + __shfl_xor_sync(full, up8 ? sx : sy, 8);
+        sz += __shfl_xor_sync(full, sz, 8);
+        sx = (up4 ? sz : sx) + __shfl_xor_sync(full, up4 ? sx : sz, 4);
+        sx += __shfl_xor_sync(full, sx, 2);
+        sx += __shfl_xor_sync(full, sx, 1);
+        const int i = up16 ? at.y : at.x;
+        if ((lane & 3) == 0 && !(up4 && up8) && i >= 0)
+            acc_add(static_cast<long long *>(up4 ? v.fz : (up8 ? v.fy : v.fx)) + i, sx);
+        for (; near; near &= near - 1)
+            near_cutoff<ENERGY, SW>(v, S, spans, nsp, kbase, q - W, (__ffs(near) - 1) << 8, q_addr, lj_addr);
     }
     if (ENERGY) {
-        // the packed sums, and the near-cutoff corrections (scalar)
-        ec += ecv.x;
-        ev += ecv.y;
         // each pair sits in both partners' lists
-        energy_add_f(v.E, G.sys, E_COUL, 0.5f * ec);
-        energy_add_f(v.E, G.sys, E_VDW, 0.5f * ev);
+        energy_add_f(v.E, G.sys, E_COUL, 0.5f * (F.ec.x + F.ec.y));
+        energy_add_f(v.E, G.sys, E_VDW, 0.5f * (F.ev.x + F.ev.y));
     }
 }
 
@@ -762,7 +927,7 @@ __global__ void __launch_bounds__(kWarps64 * 32, 2) k_pairs_fp64(DevView v) {
     int4 *s_u = reinterpret_cast<int4 *>(smem);
     HoodSpan *spans = reinterpret_cast<HoodSpan *>(s_u + v.hood_cap);
     __shared__ int2 s_queue[kWarps64][64];
-    __shared__ int2 s_nn;
+    __shared__ int4 s_nn;
     __shared__ int s_next;
     {
         const int *src = v.gspan + (size_t)blockIdx.x * kGroupSpanWords;
@@ -794,16 +959,20 @@ __global__ void __launch_bounds__(kWarps64 * 32, 2) k_pairs_fp64(DevView v) {
     int2 *queue = s_queue[warp];
     const unsigned lt = (1u << lane) - 1u;
     int head = 0, tail = 0;  // the queue holds entries head .. tail - 1 (at most 63), entry k at k & 63
-    // a unit of work: the even or the odd chunks of one atom's list, taken by
-    // the next warp that is free
+    const int q0 = pair_first(a0, G.cell), q1 = pair_first(a1, G.cell + G.ncell);
+    // a unit of work: the even or the odd chunks of a pair's list for one of
+    // its atoms, taken by the next warp that is free
     for (;;) {
         int t = lane == 0 ? atomicAdd(&s_next, 1) : 0;
         t = __shfl_sync(full, t, 0) * gridDim.y + blockIdx.y;
-        const int i = a0 + (t >> 1);
-        if (i >= a1) break;
+        const int q = q0 + (t >> 2), second = (t >> 1) & 1;
+        if (q >= q1) break;
+        const int2 ab = v.ipair[q];
+        const int i = second ? ab.y : ab.x;
+        if (i < 0) continue;
         const int4 ui = v.uf[i];
-        const int cnt = v.ncount[i];
-        const uint4 *lst4 = reinterpret_cast<const uint4 *>(v.nl16 + (size_t)i * v.stride) + lane;
+        const int cnt = v.ncount[q].x;
+        const uint4 *lst4 = reinterpret_cast<const uint4 *>(pair_list(v, q)) + lane;
         P.cur = i;
         for (int c0 = 256 * (t & 1); c0 < cnt; c0 += 512) {
             const uint4 w4 = __ldg(lst4 + c0 / 8);
@@ -811,8 +980,9 @@ __global__ void __launch_bounds__(kWarps64 * 32, 2) k_pairs_fp64(DevView v) {
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 if (c0 + 32 * u >= cnt) break;  // warp-uniform
-                const bool valid = c0 + 32 * u + lane < cnt;
                 const unsigned e = (wds[u >> 1] >> (16 * (u & 1))) & 0xffffu;
+                // not past the end, not excluded from this atom
+                const bool valid = c0 + 32 * u + lane < cnt && !((e >> second) & 1);
                 const int4 uj = s_u[valid ? e >> kEntryShift : 0];
                 const float dx = (float)(uj.x - ui.x) * ux, dy = (float)(uj.y - ui.y) * uy,
                             dz = (float)(uj.z - ui.z) * uz;
@@ -847,6 +1017,20 @@ __global__ void __launch_bounds__(kWarps64 * 32, 2) k_pairs_fp64(DevView v) {
     }
 }
 
+// Position of tile entry k in the group's frame, as stage() forms it.
+__device__ __forceinline__ void tile_position(const DevView &v, const SysDev &S, const HoodSpan *spans, int nsp, int k,
+                                              float p[3]) {
+    const int j = hood_slot(spans, nsp, k);
+    int sp = 0;
+    while (sp + 1 < nsp && spans[sp + 1].offset <= k) ++sp;
+    const int c3 = v.cell3[j];
+    const float4 D = v.dtab[v.sys_of[j] * kDtabStride + spans[sp].code0 + (((c3 >> 20) & 1023) - spans[sp].cz0)];
+    offset_in_cell(v, S, j, c3, p);
+    p[0] -= D.x;
+    p[1] -= D.y;
+    p[2] -= D.z;
+}
+
 // ---- test support: the neighbour pair set within the cutoff, exactly as
 // the reference decides it, as (larger, smaller) original indices.
 __global__ void k_collect(DevView v, int sys_sel, int *out, long long cap, unsigned long long *n_out) {
@@ -862,19 +1046,35 @@ __global__ void k_collect(DevView v, int sys_sel, int *out, long long cap, unsig
     hood_setup(v, S, v.cell3[a0], G.ncell, spans, s_n, nullptr);
     if (s_n[1] > kMaxSpans) return;
     int nsp = s_n[1];
+    const int kbase = v.gspan_n[blockIdx.x].z;
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int i = a0 + warp; i < a1; i += nw) {
-        int oi = v.orig[i];
-        int cnt = v.ncount[i];
+    const int q1 = pair_first(a1, G.cell + G.ncell);
+    for (int q = pair_first(a0, G.cell) + warp; q < q1; q += nw) {
+        const int2 ab = v.ipair[q];
+        if (ab.x < 0) continue;
+        const int cnt = v.ncount[q].x;
         for (int k = lane; k < cnt; k += 32) {
-            int j = hood_slot(spans, nsp, v.nl16[(size_t)i * v.stride + list_pos(k)] >> kEntryShift);
-            int oj = v.orig[j];
-            if (oi <= oj) continue;
-            if (!(exact_r2(v, S, i, j) < S.cut2)) continue;
-            unsigned long long p = atomicAdd(n_out, 1ull);
-            if ((long long)p < cap) {
-                out[2 * p] = oi - S.atom_off;
-                out[2 * p + 1] = oj - S.atom_off;
+            const unsigned e = pair_list(v, q)[list_pos(k)];
+            const int j = hood_slot(spans, nsp, (int)(e >> kEntryShift)), oj = v.orig[j];
+            // the entry's image of j in the group's frame
+            float tj[3];
+            tile_position(v, S, spans, nsp, (int)(e >> kEntryShift), tj);
+            for (int m = 0; m < 2; ++m) {
+                const int i = m ? ab.y : ab.x;
+                if (i < 0 || ((e >> m) & 1)) continue;
+                const int oi = v.orig[i];
+                if (oi <= oj) continue;
+                float ti[3];
+                tile_position(v, S, spans, nsp, kbase + i, ti);
+                bool near = true;
+                for (int d = 0; d < 3; ++d) near = near && fabsf(ti[d] - tj[d]) < S.halfLf[d];
+                if (!near) continue;  // another image of j, listed for the pair's other atom
+                if (!(exact_r2(v, S, i, j) < S.cut2)) continue;
+                unsigned long long p = atomicAdd(n_out, 1ull);
+                if ((long long)p < cap) {
+                    out[2 * p] = oi - S.atom_off;
+                    out[2 * p + 1] = oj - S.atom_off;
+                }
             }
         }
     }
@@ -884,10 +1084,12 @@ __global__ void k_collect(DevView v, int sys_sel, int *out, long long cap, unsig
 
 static size_t tail_bytes() { return kMaxSpans * sizeof(HoodSpan) + 4 * sizeof(int); }
 static size_t smem_build(int cap, int warps) {
-    return (size_t)cap * sizeof(float4) + (size_t)warps * 512 * sizeof(uint16_t) +
+    return (size_t)cap * sizeof(float4) + (size_t)warps * kBuildWarpWords * sizeof(uint16_t) +
            25 * (kRowCells + 1) * sizeof(int) + tail_bytes();
 }
-static size_t smem_pairs(int cap) { return (size_t)cap * (sizeof(float4) + sizeof(float2)) + tail_bytes(); }
+static size_t smem_pairs(int cap) {
+    return (size_t)(cap + kTileSpare) * (sizeof(float4) + sizeof(float2)) + tail_bytes();
+}
 static size_t smem_pairs64(int cap) { return (size_t)cap * sizeof(int4) + tail_bytes(); }
 // static shared memory of the tile kernels (displacement table and counts)
 constexpr size_t kTileStatic = 25 * kRowCells * sizeof(float4) + 16;
@@ -899,6 +1101,12 @@ constexpr size_t kTileStatic = 25 * kRowCells * sizeof(float4) + 16;
 static bool wide(size_t dynamic_smem) { return 2 * (dynamic_smem + kTileStatic + 1024) > 228 * 1024; }
 static int build_warps(int cap) { return wide(smem_build(cap, kHoodWarps)) ? 2 * kHoodWarps : kHoodWarps; }
 static int pair_warps(int cap) { return wide(smem_pairs(cap)) ? 2 * kHoodWarps : kHoodWarps; }
+
+template <int W>
+static void set_build_smem(int b) {
+    cudaFuncSetAttribute(k_build<true, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    cudaFuncSetAttribute(k_build<false, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+}
 
 template <int W>
 static void set_pairs_smem(int m) {
@@ -922,22 +1130,23 @@ void tiles_set_smem(int cap) {
     const int b = (int)smem_build(cap, bw), m = (int)smem_pairs(cap), d = (int)smem_pairs64(cap);
     const int bi = bw == kHoodWarps ? 0 : 1, pi = pw == kHoodWarps ? 0 : 1;
     std::lock_guard<std::mutex> lock(mu);
-    // launches up to 48 KB need no attribute
-    if (b > 48 * 1024 && b > seen_build[bi][dev]) {
+    // launches up to 48 KB, static shared memory included, need no attribute
+    constexpr int kFree = 48 * 1024 - (int)kTileStatic - 1024;
+    if (b > kFree && b > seen_build[bi][dev]) {
         if (bi)
-            cudaFuncSetAttribute(k_build<2 * kHoodWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+            set_build_smem<2 * kHoodWarps>(b);
         else
-            cudaFuncSetAttribute(k_build<kHoodWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+            set_build_smem<kHoodWarps>(b);
         seen_build[bi][dev] = b;
     }
-    if (m > 48 * 1024 && m > seen_pairs[pi][dev]) {
+    if (m > kFree && m > seen_pairs[pi][dev]) {
         if (pi)
             set_pairs_smem<2 * kHoodWarps>(m);
         else
             set_pairs_smem<kHoodWarps>(m);
         seen_pairs[pi][dev] = m;
     }
-    if (d > 48 * 1024 && d > seen_pairs64[dev]) {
+    if (d > kFree && d > seen_pairs64[dev]) {
         cudaFuncSetAttribute(k_pairs_fp64<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, d);
         cudaFuncSetAttribute(k_pairs_fp64<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, d);
         cudaFuncSetAttribute(k_pairs_fp64<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, d);
@@ -946,13 +1155,21 @@ void tiles_set_smem(int cap) {
     }
 }
 
+template <int W>
+static void launch_build_w(const DevView &v, cudaStream_t st) {
+    const size_t sm = smem_build(v.hood_cap, W);
+    if (v.mixed)
+        k_build<true, W><<<v.ngroups, W * 32, sm, st>>>(v);
+    else
+        k_build<false, W><<<v.ngroups, W * 32, sm, st>>>(v);
+}
+
 void launch_build(const DevView &v, cudaStream_t st) {
     if (!v.ngroups) return;
     if (build_warps(v.hood_cap) == kHoodWarps)
-        k_build<kHoodWarps><<<v.ngroups, kHoodWarps * 32, smem_build(v.hood_cap, kHoodWarps), st>>>(v);
+        launch_build_w<kHoodWarps>(v, st);
     else
-        k_build<2 * kHoodWarps>
-            <<<v.ngroups, 2 * kHoodWarps * 32, smem_build(v.hood_cap, 2 * kHoodWarps), st>>>(v);
+        launch_build_w<2 * kHoodWarps>(v, st);
 }
 
 template <int W>

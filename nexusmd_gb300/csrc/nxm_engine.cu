@@ -830,7 +830,8 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
             const SysDev &D = sysd_[s];
             ngr += (size_t)D.nc[0] * D.nc[1] * ((D.nc[2] + group_g[s] - 1) / group_g[s]);
         }
-        const size_t est = (size_t)N_ * (600 + 2 * (size_t)stride) + 12 * ((size_t)cell_off + 1) +
+        const size_t est = (size_t)N_ * (600 + (size_t)pair_stride(stride)) +
+                           (20 + (size_t)pair_stride(stride)) * ((size_t)cell_off + 2) +
                            ngr * (sizeof(CellGroup) + 4 * (size_t)kGroupSpanWords + 8) +
                            (size_t)S * (kDtabStride * sizeof(float4) + 24 * E_SLOTS + sizeof(SysDev)) +
                            8 * (size_t)cg_total + 56 * nb + 56 * na + 60 * nt + 88 * nx + 16 * (size_t)roff +
@@ -869,7 +870,9 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
     hood_cap = (hood_cap + 31) / 32 * 32;
     if (hood_cap > 8191) return "neighbourhood too dense for 16-bit list entries";
     v_.hood_cap = hood_cap;
-    v_.nl16 = dalloc<uint16_t>((size_t)N_ * stride);
+    const size_t npair = (size_t)pair_first(N_, cell_off) + 1;
+    v_.nl16 = dalloc<uint16_t>(npair * pair_stride(stride));
+    v_.ipair = dalloc<int2>(npair);
     {
         // groups of G consecutive cells along each z-row of every system
         std::vector<CellGroup> gr;
@@ -889,11 +892,11 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
         v_.ngroups = (int)gr.size();
         v_.groups = dalloc<CellGroup>(gr.size());
         v_.gspan = dalloc<int>(gr.size() * (size_t)kGroupSpanWords);
-        v_.gspan_n = dalloc<int2>(gr.size());
+        v_.gspan_n = dalloc<int4>(gr.size());
         cudaMemcpyAsync(v_.groups, gr.data(), sizeof(CellGroup) * gr.size(), cudaMemcpyHostToDevice, st_copy_);
     }
     tiles_set_smem(hood_cap);
-    v_.ncount = dalloc<int>(N_);
+    v_.ncount = dalloc<int2>(npair);
     v_.dtab = dalloc<float4>((size_t)S * kDtabStride);
     v_.xref = dalloc<double>(3 * (size_t)N_);
     v_.oref = dalloc<float4>(N_);

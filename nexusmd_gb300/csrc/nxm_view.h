@@ -45,14 +45,16 @@ struct DevView {
     int total_cells;
     int *cell_key, *cell_count, *cell_start, *cell_fill;
     int *new_orig;
-    uint16_t *nl16;      // per-atom list of indices into the cell's staged neighbourhood
-    int *ncount;
-    int stride;
+    int2 *ipair;         // pairs of atoms (slots) that share a list: cell c's from pair_first(cell_start[c], c); second
+                         // -1: an atom alone, both -1: an unused place
+    uint16_t *nl16;      // per-pair list of indices into the group's staged neighbourhood
+    int2 *ncount;        // per pair: entries, and one bit per 256-entry chunk that holds one excluded from one atom
+    int stride;          // an atom's list capacity (a pair's: pair_stride)
     struct CellGroup *groups;  // blocks of the tile kernels: runs of cells along z
     int ngroups;
     int hood_cap;        // capacity of a staged neighbourhood (atoms)
     int *gspan;          // [ngroups][kGroupSpanWords]: each group's neighbourhood spans, written by the list build
-    int2 *gspan_n;       // [ngroups]: (atoms, spans) of that neighbourhood
+    int4 *gspan_n;       // [ngroups]: atoms and spans of that neighbourhood, tile index of slot 0
     float4 *dtab;        // [S][kDtabStride] cell-image displacement per code
     float2 *cgrid;       // per system and axis, per cell: corner's PME grid coordinate (int part, fraction)
     double *xref;        // [3][N] positions at the last rebuild (mixed: as fix40 integers)
@@ -93,6 +95,15 @@ struct DevView {
     double *snap_x, *snap_v, *snap_f;
     double skin_half2;   // (skin/2)^2; 0 disables the displacement check
 };
+
+// First place in DevView::ipair of the pairs of cell c, whose first slot is
+// `start`: room for (n + 1) / 2 pairs of its n atoms, at most one place of
+// which stays unused.
+__host__ __device__ __forceinline__ int pair_first(int start, int c) { return (start + c) >> 1; }
+
+// Entries a pair's list has room for: the union of any two lists within an
+// atom's capacity, filled up to a multiple of 32; whole 256-entry chunks.
+__host__ __device__ __forceinline__ int pair_stride(int stride) { return 2 * stride + 256; }
 
 // Context creation: the exclusion sets built on the device
 // (k_exclusions_build.cu).  deg, xdeg, afill and xfill are consecutive runs
