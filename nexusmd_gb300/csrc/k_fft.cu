@@ -17,12 +17,15 @@
 //    kernel convolves, one block per x-plane does y and then z (inverse);
 //  * line path (5 kernels): z, y, x, y, z, each kernel over tiles of lines --
 //    for planes too large for shared memory, and for the no-allocation entry.
+// The two are the faster ones in turn (one system, warm L2): 100^3 plane 41,
+// line 48 us; 180^3 181 and 107; the autotuner times both.
 // Every pass has its radix fixed at compile time and reads its twiddles from
 // a shared-memory copy of the axis's table; lines in shared memory have an odd
 // stride (in complex words) so that column accesses do not conflict on banks.
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "nxm_fft.h"
 #include "nxm_view.h"
@@ -371,13 +374,14 @@ __device__ __forceinline__ void z_inverse(typename Cx<C>::R *out, int nreal, int
 // Shared memory: twiddles of y and z (twcap), the plane Q as Kh columns of
 // length K1 with odd stride ldq (qcap), two scratch buffers of `scr` words.
 
-template <typename C, typename Acc>
-__global__ void __launch_bounds__(1024) k_fft_plane_fwd(DevView v, const FftSysDev *fs, const FftWork *work,
+template <typename C, typename Acc, bool ONE>
+__global__ void __launch_bounds__(1024) k_fft_plane_fwd(const __grid_constant__ DevView v, const FftSysDev *fs,
+                            const __grid_constant__ FftSysDev one, const FftWork *work,
                                                         int twcap, int qcap, int scr) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *twy = reinterpret_cast<C *>(smem_raw);
-    FftWork w = work[blockIdx.x];
-    const FftSysDev &F = fs[w.sys];
+    const FftWork w = ONE ? FftWork{0, (int)blockIdx.x} : work[blockIdx.x];
+    const FftSysDev &F = ONE ? one : fs[w.sys];
     const int K1 = F.K[1], K2 = F.K[2], Kh = F.Kh, x = w.unit;
     const int ldq = K1 | 1, ldz = K2 | 1;
     C *twz = twy + K1;
@@ -410,14 +414,15 @@ __global__ void __launch_bounds__(1024) k_fft_plane_fwd(DevView v, const FftSysD
     }
 }
 
-template <typename C>
-__global__ void __launch_bounds__(1024) k_fft_plane_inv(DevView v, const FftSysDev *fs, const FftWork *work,
+template <typename C, bool ONE>
+__global__ void __launch_bounds__(1024) k_fft_plane_inv(const __grid_constant__ DevView v, const FftSysDev *fs,
+                            const __grid_constant__ FftSysDev one, const FftWork *work,
                                                         int twcap, int qcap, int scr) {
     using T = typename Cx<C>::R;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *twy = reinterpret_cast<C *>(smem_raw);
-    FftWork w = work[blockIdx.x];
-    const FftSysDev &F = fs[w.sys];
+    const FftWork w = ONE ? FftWork{0, (int)blockIdx.x} : work[blockIdx.x];
+    const FftSysDev &F = ONE ? one : fs[w.sys];
     const int K1 = F.K[1], K2 = F.K[2], Kh = F.Kh, x = w.unit;
     const int ldq = K1 | 1, ldz = K2 | 1;
     C *twz = twy + K1;
@@ -451,166 +456,395 @@ __global__ void __launch_bounds__(1024) k_fft_plane_inv(DevView v, const FftSysD
 }
 
 // ================= line path: tiles of lines per block =================
+// A block transforms a tile of lines with the elements in registers between
+// passes where they can be: the first pass reads its elements from global
+// memory, the last stores them there (or hands them on), and only what
+// changes threads between two passes goes through shared memory.  Bound by
+// the latency of that chain (the grid stays in L2): per kernel one or two
+// exchanges and their barriers instead of a shared-memory round trip and a
+// barrier before, between and after the passes (100^3: 14 -> 8 M warp
+// instructions).  Per convolution, line path: 180^3 136 -> 107 us, 64x96x125
+// 47 -> 39, a batch of 32 grids of 30^3 to 60^3 103 -> 85, FP64 at 64^3
+// 78 -> 64; with the plane path 32^3 24.6 -> 20.5, 100^3 43.0 -> 40.9.
+//
+// y and x: the lines are the half spectrum's columns, numbered along memory,
+// and lane order runs over consecutive lines (item = j * L + line, L a power
+// of two), so every access is a run of L neighbouring words and no index
+// needs a division.  z: lane order runs along the line (item = line * m + j).
 // Shared memory: the axis's twiddles (kmax words), two line buffers.
 
-// z forward: L real lines (L/2 complex) per block.
-template <typename C, typename Acc>
-__global__ void __launch_bounds__(256) k_fft_z_fwd(DevView v, const FftSysDev *fs, const FftWork *work, int L,
+// The axis's twiddles on their way to shared memory: the thread's first word
+// is asked for before the first pass (which needs none) and stored after it,
+// so its latency passes beside that pass's loads.
+template <typename C>
+struct Twiddles {
+    const C *src;
+    C *dst;
+    int n;
+    C first;
+    __device__ __forceinline__ Twiddles(C *dst_, const DevView &v, int off, int n_)
+        : src(static_cast<const C *>(v.twiddle) + off), dst(dst_), n(n_) {
+        first = src[min((int)threadIdx.x, n - 1)];
+    }
+    __device__ __forceinline__ void store() const {
+        if ((int)threadIdx.x < n) dst[threadIdx.x] = first;
+        for (int i = threadIdx.x + blockDim.x; i < n; i += blockDim.x) dst[i] = src[i];
+    }
+};
+
+// Calls f(R) with the radix as a compile-time constant.
+template <typename F>
+__device__ __forceinline__ void with_radix(int R, F f) {
+    switch (R) {
+        case 10: f(std::integral_constant<int, 10>{}); break;
+        case 9: f(std::integral_constant<int, 9>{}); break;
+        case 8: f(std::integral_constant<int, 8>{}); break;
+        case 6: f(std::integral_constant<int, 6>{}); break;
+        case 4: f(std::integral_constant<int, 4>{}); break;
+        case 3: f(std::integral_constant<int, 3>{}); break;
+        case 2: f(std::integral_constant<int, 2>{}); break;
+        default: f(std::integral_constant<int, 5>{}); break;
+    }
+}
+
+// A butterfly's inputs times W^(r k step) (conjugated for the inverse).
+template <typename C, int R, bool INV>
+__device__ __forceinline__ void twiddle(C *v, int k, int step, const C *tw) {
+    if (k) {
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+            C w = tw[r * k * step];
+            if (INV) w.y = -w.y;
+            v[r] = cmul(v[r], w);
+        }
+    }
+}
+
+// The lines of a block and how its threads' items map to (line, butterfly).
+template <bool ALONG>
+struct Tile {
+    int nl, lg, ld;  // lines present; log2 of the tile's lines (ALONG false); line stride in shared memory
+    __device__ __forceinline__ int items(int m) const { return ALONG ? nl * m : m << lg; }
+    // false: no such line
+    __device__ __forceinline__ bool at(int item, int m, float inv_m, int &l, int &j) const {
+        if (ALONG) {
+            l = quot(item, inv_m);
+            j = item - l * m;
+            return true;
+        }
+        l = item & ((1 << lg) - 1);
+        j = item >> lg;
+        return l < nl;
+    }
+};
+
+// Pass p (not the last) of P: inputs from load(line, element), or from `src`
+// for a later pass; outputs to dst, where the next pass finds them.
+template <typename C, bool INV, bool ALONG, typename Load>
+__device__ __forceinline__ void pass_to_smem(const Tile<ALONG> &T, const FftPasses &P, int p, C *dst, const C *tw,
+                                             Load load) {
+    const int m = P.m[p], Ns = P.Ns[p], step = P.step[p];
+    const float inv_m = P.inv_m[p], inv_ns = P.inv_ns[p];
+    with_radix(P.R[p], [&](auto radix) {
+        constexpr int R = decltype(radix)::value;
+        for (int it = threadIdx.x; it < T.items(m); it += blockDim.x) {
+            int l, j;
+            if (!T.at(it, m, inv_m, l, j)) continue;
+            const int jq = quot(j, inv_ns), k = j - jq * Ns;
+            C v[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[r] = load(l, j + r * m);
+            twiddle<C, R, INV>(v, k, step, tw);
+            small_dft<C, R>(v, (typename Cx<C>::R)(INV ? 1 : -1));
+            C *d = dst + l * T.ld + jq * Ns * R + k;
+#pragma unroll
+            for (int r = 0; r < R; ++r) d[r * Ns] = v[r];
+        }
+    });
+}
+
+// The last pass of P: butterfly j's outputs are the line's elements j + r m,
+// handed to store(line, element, value).
+template <typename C, bool INV, bool ALONG, typename Load, typename Store>
+__device__ __forceinline__ void last_pass(const Tile<ALONG> &T, const FftPasses &P, const C *tw, Load load,
+                                          Store store) {
+    const int p = P.np - 1, m = P.m[p], step = P.step[p];
+    const float inv_m = P.inv_m[p];
+    with_radix(P.R[p], [&](auto radix) {
+        constexpr int R = decltype(radix)::value;
+        for (int it = threadIdx.x; it < T.items(m); it += blockDim.x) {
+            int l, j;
+            if (!T.at(it, m, inv_m, l, j)) continue;
+            C v[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[r] = load(l, j + r * m);
+            if (p) twiddle<C, R, INV>(v, j, step, tw);
+            small_dft<C, R>(v, (typename Cx<C>::R)(INV ? 1 : -1));
+#pragma unroll
+            for (int r = 0; r < R; ++r) store(l, j + r * m, v[r]);
+        }
+    });
+}
+
+// All passes of P over the tile: load and store as above; a and b are the
+// block's line buffers.  `whole`: from the first pass on; otherwise its
+// outputs (and the twiddles) are in shared memory already, behind a barrier.
+template <typename C, bool INV, bool ALONG, typename Load, typename Store>
+__device__ __forceinline__ void tile_fft(const Tile<ALONG> &T, const FftPasses &P, C *a, C *b, const Twiddles<C> &twl,
+                                         bool whole, Load load, Store store) {
+    const int np = P.np;
+    const C *tw = twl.dst;
+    if (np == 1) {
+        last_pass<C, INV>(T, P, tw, load, store);
+        return;
+    }
+    if (whole) {
+        pass_to_smem<C, INV>(T, P, 0, a, tw, load);
+        twl.store();
+        __syncthreads();
+    }
+    C *src = a, *dst = b;
+    auto from = [&](int l, int e) { return src[l * T.ld + e]; };
+    for (int p = 1; p < np - 1; ++p) {
+        pass_to_smem<C, INV>(T, P, p, dst, tw, from);
+        __syncthreads();
+        C *t = src;
+        src = dst;
+        dst = t;
+    }
+    last_pass<C, INV>(T, P, tw, from, store);
+}
+
+// z forward: L real lines (L/2 complex) per block; pairs of lines as one
+// complex line, separated after the transform (z_forward above).
+template <typename C, typename Acc, bool ONE>
+__global__ void __launch_bounds__(256) k_fft_z_fwd(const __grid_constant__ DevView v, const FftSysDev *fs,
+                            const __grid_constant__ FftSysDev one, const FftWork *work, int L,
                                                    int kmax) {
+    using T = typename Cx<C>::R;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *tw = reinterpret_cast<C *>(smem_raw);
-    FftWork w = work[blockIdx.x];
-    const FftSysDev &F = fs[w.sys];
+    const FftWork w = ONE ? FftWork{0, (int)blockIdx.x} : work[blockIdx.x];
+    const FftSysDev &F = ONE ? one : fs[w.sys];
     const int n = F.K[2], Kh = F.Kh, ld = n | 1;
     const int l0 = w.unit * L, nl = min(L, F.K[0] * F.K[1] - l0);
     C *a = tw + kmax;
     C *b = a + (L >> 1) * ld;
-    load_tw(tw, v, F.tw[2], n);
+    const Twiddles<C> twl(tw, v, F.tw[2], n);
     const Acc *acc = static_cast<const Acc *>(v.grid_acc) + F.roff + (long long)l0 * n;
     C *out = static_cast<C *>(v.grid_cplx) + F.coff + (long long)l0 * Kh;
-    z_forward<C, Acc>(acc, nl, (nl + 1) >> 1, n, Kh, a, b, ld, F, tw, [&](int p, int k, C xa, C xb, bool hb) {
-        out[(long long)(2 * p) * Kh + k] = xa;
-        if (hb) out[(long long)(2 * p + 1) * Kh + k] = xb;
-    });
-}
-
-// y: columns of the half spectrum for fixed x, `cols` consecutive kz.
-template <typename C, bool INV>
-__global__ void __launch_bounds__(256) k_fft_y(DevView v, const FftSysDev *fs, const FftWork *work, int cols,
-                                               int kmax) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *tw = reinterpret_cast<C *>(smem_raw);
-    FftWork w = work[blockIdx.x];
-    const FftSysDev &F = fs[w.sys];
-    const int n = F.K[1], Kh = F.Kh, ld = n | 1;
-    const int chunks = (Kh + cols - 1) / cols;
-    const int x = w.unit / chunks, z0 = (w.unit - x * chunks) * cols;
-    const int nc = min(cols, Kh - z0);
-    C *a = tw + kmax;
-    C *b = a + cols * ld;
-    load_tw(tw, v, F.tw[1], n);
-    C *g = static_cast<C *>(v.grid_cplx) + F.coff + (long long)x * F.K[1] * Kh + z0;
-    const float inv_c = 1.0f / (float)nc;
-    // smem line c holds column z0 + c
-    rounds<kRounds>(
-        n * nc,
-        [&](int e) {
-            int y = quot(e, inv_c);
-            return g[(long long)y * Kh + e - y * nc];
+    const Tile<true> tile{(nl + 1) >> 1, 0, ld};
+    // the transform's result in order in b (two passes) or a (one or three)
+    C *res = F.ax[2].np & 1 ? a : b;
+    tile_fft<C, false>(
+        tile, F.ax[2], a, b, twl, true,
+        [&](int l, int z) {
+            const int la = 2 * l, lb = min(la + 1, nl - 1);
+            const Acc ga = __ldcs(acc + (long long)la * n + z);
+            const Acc gb = __ldcs(acc + (long long)lb * n + z);
+            return Cx<C>::mk((T)grid_value(ga), la + 1 < nl ? (T)grid_value(gb) : (T)0);
         },
-        [&](int e, C val) {
-            int y = quot(e, inv_c);
-            a[(e - y * nc) * ld + y] = val;
-        });
+        [&](int l, int k, C val) { res[l * ld + k] = val; });
     __syncthreads();
-    int ldr;
-    C *res = line_fft<C, INV>(a, ld, nullptr, 0, b, a, ld, n, nc, F.ax[1], tw, &ldr);
-    for (int e = threadIdx.x; e < n * nc; e += blockDim.x) {
-        int y = quot(e, inv_c), c = e - y * nc;
-        g[(long long)y * Kh + c] = res[c * ldr + y];
+    const float inv_kh = 1.0f / (float)Kh;
+    for (int e = threadIdx.x; e < tile.nl * Kh; e += blockDim.x) {
+        const int p = quot(e, inv_kh), k = e - p * Kh;
+        const C z = res[p * ld + k];
+        const C zc = res[p * ld + (k == 0 ? 0 : n - k)];
+        out[(long long)(2 * p) * Kh + k] = Cx<C>::mk((T)0.5 * (z.x + zc.x), (T)0.5 * (z.y - zc.y));
+        if (2 * p + 1 < nl)
+            out[(long long)(2 * p + 1) * Kh + k] = Cx<C>::mk((T)0.5 * (z.y + zc.y), (T)0.5 * (zc.x - z.x));
     }
 }
 
-// x: forward, convolution with the influence function, energy, inverse.
-// Used by both paths.
-template <typename C, typename ET>
-__global__ void __launch_bounds__(256) k_fft_x_conv(DevView v, const FftSysDev *fs, const FftWork *work, int cols,
+// y: `cols` columns of the half spectrum per block, column l = x Kh + kz.
+template <typename C, bool INV, bool ONE>
+__global__ void __launch_bounds__(256) k_fft_y(const __grid_constant__ DevView v, const FftSysDev *fs,
+                            const __grid_constant__ FftSysDev one, const FftWork *work, int cols,
+                                               int kmax) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *tw = reinterpret_cast<C *>(smem_raw);
+    const FftWork w = ONE ? FftWork{0, (int)blockIdx.x} : work[blockIdx.x];
+    const FftSysDev &F = ONE ? one : fs[w.sys];
+    const int n = F.K[1], Kh = F.Kh, ld = n | 1;
+    const int l0 = w.unit * cols, nl = min(cols, F.K[0] * Kh - l0);
+    C *a = tw + kmax;
+    C *b = a + cols * ld;
+    const Twiddles<C> twl(tw, v, F.tw[1], n);
+    C *g = static_cast<C *>(v.grid_cplx) + F.coff;
+    const Tile<false> tile{nl, __ffs(cols) - 1, ld};
+    // a thread's items are all of one column (the block's threads are a
+    // multiple of cols)
+    const int col = l0 + min((int)threadIdx.x & (cols - 1), nl - 1);
+    const int x = quot(col, 1.0f / (float)Kh);
+    C *line = g + (long long)x * n * Kh + (col - x * Kh);
+    tile_fft<C, INV>(
+        tile, F.ax[1], a, b, twl, true, [&](int, int y) { return line[(long long)y * Kh]; },
+        [&](int, int y, C val) { line[(long long)y * Kh] = val; });
+}
+
+// x: forward, convolution with the influence function, energy, inverse, on
+// `cols` columns l = y Kh + kz per block (consecutive in memory).  The
+// forward transform's last pass leaves butterfly j the elements j + r m,
+// which are what butterfly j of the inverse's first pass takes when the
+// inverse runs the radices in reverse: spectrum and product stay in
+// registers.  Used by both paths.
+template <typename C, typename ET, bool ONE>
+__global__ void __launch_bounds__(256) k_fft_x_conv(const __grid_constant__ DevView v, const FftSysDev *fs,
+                            const __grid_constant__ FftSysDev one, const FftWork *work, int cols,
                                                     int kmax, int energy) {
     using T = typename Cx<C>::R;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *tw = reinterpret_cast<C *>(smem_raw);
-    FftWork w = work[blockIdx.x];
-    const FftSysDev &F = fs[w.sys];
+    const FftWork w = ONE ? FftWork{0, (int)blockIdx.x} : work[blockIdx.x];
+    const FftSysDev &F = ONE ? one : fs[w.sys];
     const int n = F.K[0], K1 = F.K[1], Kh = F.Kh, ld = n | 1;
-    const int chunks = (Kh + cols - 1) / cols;
-    const int y = w.unit / chunks, z0 = (w.unit - y * chunks) * cols;
-    const int nc = min(cols, Kh - z0);
+    const int l0 = w.unit * cols, nl = min(cols, K1 * Kh - l0);
     C *a = tw + kmax;
     C *b = a + cols * ld;
-    load_tw(tw, v, F.tw[0], n);
+    const Twiddles<C> twl(tw, v, F.tw[0], n);
     const long long xstride = (long long)K1 * Kh;
-    C *g = static_cast<C *>(v.grid_cplx) + F.coff + (long long)y * Kh + z0;
-    const float inv_c = 1.0f / (float)nc, inv_n = 1.0f / (float)n;
-    rounds<kRounds>(
-        n * nc,
-        [&](int e) {
-            int x = quot(e, inv_c);
-            return g[x * xstride + e - x * nc];
-        },
-        [&](int e, C val) {
-            int x = quot(e, inv_c);
-            a[(e - x * nc) * ld + x] = val;
-        });
-    __syncthreads();
-    int ldr;
-    C *res = line_fft<C, false>(a, ld, nullptr, 0, b, a, ld, n, nc, F.ax[0], tw, &ldr);
-    C *other = res == a ? b : a;
-    const ET *et = static_cast<const ET *>(v.eterm) + F.coff + (long long)y * Kh + z0;
+    const int mine = min((int)threadIdx.x & (cols - 1), nl - 1), col = l0 + mine;
+    C *g = static_cast<C *>(v.grid_cplx) + F.coff + col;
+    const ET *et = static_cast<const ET *>(v.eterm) + F.coff + col;
+    const int kz = col - quot(col, 1.0f / (float)Kh) * Kh;
+    // half spectrum: planes kz = 0 and kz = K2/2 (even K2) appear once; E = sum / 2
+    const bool once = kz == 0 || 2 * kz == F.K[2];
+    const Tile<false> tile{nl, __ffs(cols) - 1, ld};
+    const FftPasses &P = F.ax[0], &Q = F.axi;
+    const int np = P.np;
+    auto global = [&](int, int x) { return g[x * xstride]; };
+    C *src = a, *dst = b;
+    auto from = [&](int l, int e) { return src[l * ld + e]; };
+    if (np > 1) {
+        pass_to_smem<C, false>(tile, P, 0, a, tw, global);
+        twl.store();
+        for (int p = 1; p < np - 1; ++p) {
+            __syncthreads();
+            pass_to_smem<C, false>(tile, P, p, dst, tw, from);
+            C *t = src;
+            src = dst;
+            dst = t;
+        }
+    }
     // the energy in fixed point per element: its sum is the same whatever
     // the column blocking (an autotuned launch shape) groups together
     long long esum = 0;
-    rounds<kRounds>(
-        n * nc,
-        [&](int e) {
-            int c = quot(e, inv_n);
-            return (T)et[(e - c * n) * xstride + c];
-        },
-        [&](int e, T f) {
-            int c = quot(e, inv_n), kx = e - c * n;
-            int kz = z0 + c;
-            C s = res[c * ldr + kx];
-            if (energy) {
-                // half spectrum: planes kz = 0 and kz = K2/2 (even K2) appear
-                // once; E = sum / 2
-                const bool once = kz == 0 || 2 * kz == F.K[2];
-                esum += element_energy(f, s, once);
+    {
+        const int p = np - 1, m = P.m[p], step = P.step[p];
+        with_radix(P.R[p], [&](auto radix) {
+            constexpr int R = decltype(radix)::value;
+            // the influence function's values of the thread's next butterfly
+            // come in beside the barrier (and beside the butterfly before)
+            T f[R];
+            auto fetch = [&](int it) {
+                int l, j;
+                if (it < tile.items(m) && tile.at(it, m, 0.f, l, j)) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) f[r] = (T)et[(j + r * m) * xstride];
+                }
+            };
+            fetch(threadIdx.x);
+            if (np > 1) __syncthreads();
+            for (int it = threadIdx.x; it < tile.items(m); it += blockDim.x) {
+                int l, j;
+                if (!tile.at(it, m, 0.f, l, j)) continue;
+                C v[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) v[r] = np > 1 ? from(l, j + r * m) : global(l, j + r * m);
+                if (p) twiddle<C, R, false>(v, j, step, tw);
+                small_dft<C, R>(v, (T)-1);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (energy) esum += element_energy(f[r], v[r], once);
+                    v[r] = Cx<C>::mk(v[r].x * f[r], v[r].y * f[r]);
+                }
+                fetch(it + blockDim.x);
+                small_dft<C, R>(v, (T)1);
+                if (np > 1) {
+                    C *d = dst + l * ld + j * R;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) d[r] = v[r];
+                } else {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) g[(j + r * m) * xstride] = v[r];
+                }
             }
-            res[c * ldr + kx] = Cx<C>::mk(s.x * f, s.y * f);
         });
-    __syncthreads();
-    C *fin = line_fft<C, true>(res, ldr, nullptr, 0, other, res, ld, n, nc, F.ax[0], tw, &ldr);
-    for (int e = threadIdx.x; e < n * nc; e += blockDim.x) {
-        int x = quot(e, inv_c), c = e - x * nc;
-        g[x * xstride + c] = fin[c * ldr + x];
+    }
+    if (np > 1) {
+        __syncthreads();
+        tile_fft<C, true>(tile, Q, dst, src, twl, false, global, [&](int, int x, C val) { g[x * xstride] = val; });
     }
     if (energy) energy_add_fixed(v.E, w.sys, E_RECIP, esum);
 }
 
-// z inverse: L real output lines per block.
-template <typename C>
-__global__ void __launch_bounds__(256) k_fft_z_inv(DevView v, const FftSysDev *fs, const FftWork *work, int L,
+// z inverse: L real output lines per block (z_inverse above).
+template <typename C, bool ONE>
+__global__ void __launch_bounds__(256) k_fft_z_inv(const __grid_constant__ DevView v, const FftSysDev *fs,
+                            const __grid_constant__ FftSysDev one, const FftWork *work, int L,
                                                    int kmax) {
     using T = typename Cx<C>::R;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *tw = reinterpret_cast<C *>(smem_raw);
-    FftWork w = work[blockIdx.x];
-    const FftSysDev &F = fs[w.sys];
+    const FftWork w = ONE ? FftWork{0, (int)blockIdx.x} : work[blockIdx.x];
+    const FftSysDev &F = ONE ? one : fs[w.sys];
     const int n = F.K[2], Kh = F.Kh, ld = n | 1;
     const int l0 = w.unit * L, nl = min(L, F.K[0] * F.K[1] - l0);
     C *a = tw + kmax;
     C *b = a + (L >> 1) * ld;
-    load_tw(tw, v, F.tw[2], n);
+    const Twiddles<C> twl(tw, v, F.tw[2], n);
     const C *in = static_cast<const C *>(v.grid_cplx) + F.coff + (long long)l0 * Kh;
     T *out = static_cast<T *>(v.grid_real) + F.roff + (long long)l0 * n;
-    z_inverse<C>(out, nl, (nl + 1) >> 1, n, Kh, a, b, ld, F, tw,
-                 [&](int p, int kk, int second) { return in[(long long)(2 * p + second) * Kh + kk]; });
+    const Tile<true> tile{(nl + 1) >> 1, 0, ld};
+    tile_fft<C, true>(
+        tile, F.ax[2], a, b, twl, true,
+        [&](int l, int k) {
+            const bool upper = k >= Kh, two = 2 * l + 1 < nl;
+            const int kk = upper ? n - k : k;
+            C A = in[(long long)(2 * l) * Kh + kk];
+            C B = in[(long long)(two ? 2 * l + 1 : 2 * l) * Kh + kk];
+            if (!two) B = Cx<C>::mk((T)0, (T)0);
+            if (upper) {
+                A.y = -A.y;
+                B.y = -B.y;
+            }
+            return Cx<C>::mk(A.x - B.y, A.y + B.x);
+        },
+        [&](int l, int z, C val) {
+            out[(long long)(2 * l) * n + z] = val.x;
+            if (2 * l + 1 < nl) out[(long long)(2 * l + 1) * n + z] = val.y;
+        });
+}
+
+// One system (ONE): its geometry comes as a kernel parameter and a block's
+// unit is its index, which takes two dependent global loads out of the
+// start of each of these latency-bound kernels.
+template <typename C, typename Acc, typename ET, bool ONE>
+static void run(const DevView &v, const FftPlan &p, int energy, cudaStream_t st) {
+    const FftSysDev &F = ONE ? p.hsys[0] : FftSysDev{};
+    if (p.plane) {
+        k_fft_plane_fwd<C, Acc, ONE>
+            <<<p.npl, p.plane_threads, p.smem_plane, st>>>(v, p.dsys, F, p.pwork, p.twcap, p.qcap, p.scr);
+        k_fft_x_conv<C, ET, ONE><<<p.nx, p.cthreads, p.smem_x, st>>>(v, p.dsys, F, p.xwork, p.cols, p.kmax, energy);
+        k_fft_plane_inv<C, ONE>
+            <<<p.npl, p.plane_threads, p.smem_plane, st>>>(v, p.dsys, F, p.pwork, p.twcap, p.qcap, p.scr);
+        return;
+    }
+    k_fft_z_fwd<C, Acc, ONE><<<p.nz, p.zthreads, p.smem_z, st>>>(v, p.dsys, F, p.zwork, p.zlines, p.kmax);
+    k_fft_y<C, false, ONE><<<p.ny, p.cthreads, p.smem_y, st>>>(v, p.dsys, F, p.ywork, p.cols, p.kmax);
+    k_fft_x_conv<C, ET, ONE><<<p.nx, p.cthreads, p.smem_x, st>>>(v, p.dsys, F, p.xwork, p.cols, p.kmax, energy);
+    k_fft_y<C, true, ONE><<<p.ny, p.cthreads, p.smem_y, st>>>(v, p.dsys, F, p.ywork, p.cols, p.kmax);
+    k_fft_z_inv<C, ONE><<<p.nz, p.zthreads, p.smem_z, st>>>(v, p.dsys, F, p.zwork, p.zlines, p.kmax);
 }
 
 template <typename C, typename Acc, typename ET>
 static void run(const DevView &v, const FftPlan &p, int energy, cudaStream_t st) {
     if (p.nz == 0) return;
-    if (p.plane) {
-        k_fft_plane_fwd<C, Acc><<<p.npl, p.plane_threads, p.smem_plane, st>>>(v, p.dsys, p.pwork, p.twcap, p.qcap,
-                                                                            p.scr);
-        k_fft_x_conv<C, ET><<<p.nx, 256, p.smem_x, st>>>(v, p.dsys, p.xwork, p.cols, p.kmax, energy);
-        k_fft_plane_inv<C><<<p.npl, p.plane_threads, p.smem_plane, st>>>(v, p.dsys, p.pwork, p.twcap, p.qcap, p.scr);
-        return;
-    }
-    k_fft_z_fwd<C, Acc><<<p.nz, 256, p.smem_z, st>>>(v, p.dsys, p.zwork, p.zlines, p.kmax);
-    k_fft_y<C, false><<<p.ny, 256, p.smem_y, st>>>(v, p.dsys, p.ywork, p.cols, p.kmax);
-    k_fft_x_conv<C, ET><<<p.nx, 256, p.smem_x, st>>>(v, p.dsys, p.xwork, p.cols, p.kmax, energy);
-    k_fft_y<C, true><<<p.ny, 256, p.smem_y, st>>>(v, p.dsys, p.ywork, p.cols, p.kmax);
-    k_fft_z_inv<C><<<p.nz, 256, p.smem_z, st>>>(v, p.dsys, p.zwork, p.zlines, p.kmax);
+    if (p.hsys.size() == 1)
+        run<C, Acc, ET, true>(v, p, energy, st);
+    else
+        run<C, Acc, ET, false>(v, p, energy, st);
 }
 
 void launch_fft_convolve(const DevView &v, const FftPlan &p, int energy, cudaStream_t st) {
@@ -646,13 +880,35 @@ void fft_passes(int n, FftPasses &P) {
     }
 }
 
+void fft_passes_reversed(int n, const FftPasses &P, FftPasses &Q) {
+    Q = FftPasses{};
+    Q.np = P.np;
+    int Ns = 1;
+    for (int p = 0; p < P.np; ++p) {
+        Q.R[p] = P.R[P.np - 1 - p];
+        Q.Ns[p] = Ns;
+        Q.m[p] = n / Q.R[p];
+        Q.step[p] = n / (Ns * Q.R[p]);
+        Q.inv_m[p] = 1.0f / (float)Q.m[p];
+        Q.inv_ns[p] = 1.0f / (float)Ns;
+        Ns *= Q.R[p];
+    }
+}
+
+int fft_line_threads(const std::vector<FftSysDev> &sys, int d, int lines) {
+    int most = 32;
+    for (const FftSysDev &F : sys)
+        for (int p = 0; p < F.ax[d].np; ++p) most = std::max(most, lines * F.ax[d].m[p]);
+    return std::min(256, (most + 31) / 32 * 32);
+}
+
 // Raises a kernel's dynamic shared-memory limit.  The limit is a per-kernel
 // attribute shared by every context (and plan) of the process on a device:
 // it is only ever raised, so a plan with smaller lines cannot lower it under
 // another one.  `slot` names the kernel (one per kernel and precision).
 static void raise_smem(const void *kernel, int slot, size_t bytes) {
     static std::mutex mu;
-    static size_t seen[16][kMaxSmemDevices] = {};
+    static size_t seen[32][kMaxSmemDevices] = {};
     if (bytes <= 48 * 1024) return;  // launches up to 48 KB need no attribute
     int dev = 0;
     cudaGetDevice(&dev);
@@ -663,16 +919,16 @@ static void raise_smem(const void *kernel, int slot, size_t bytes) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-template <typename C, typename Acc, typename ET>
+template <typename C, typename Acc, typename ET, bool ONE>
 static void raise_all(const FftPlan &p, int base) {
-    raise_smem((const void *)k_fft_z_fwd<C, Acc>, base + 0, p.smem_z);
-    raise_smem((const void *)k_fft_z_inv<C>, base + 1, p.smem_z);
-    raise_smem((const void *)k_fft_y<C, false>, base + 2, p.smem_y);
-    raise_smem((const void *)k_fft_y<C, true>, base + 3, p.smem_y);
-    raise_smem((const void *)k_fft_x_conv<C, ET>, base + 4, p.smem_x);
+    raise_smem((const void *)k_fft_z_fwd<C, Acc, ONE>, base + 0, p.smem_z);
+    raise_smem((const void *)k_fft_z_inv<C, ONE>, base + 1, p.smem_z);
+    raise_smem((const void *)k_fft_y<C, false, ONE>, base + 2, p.smem_y);
+    raise_smem((const void *)k_fft_y<C, true, ONE>, base + 3, p.smem_y);
+    raise_smem((const void *)k_fft_x_conv<C, ET, ONE>, base + 4, p.smem_x);
     if (p.plane_ok) {
-        raise_smem((const void *)k_fft_plane_fwd<C, Acc>, base + 5, p.smem_plane);
-        raise_smem((const void *)k_fft_plane_inv<C>, base + 6, p.smem_plane);
+        raise_smem((const void *)k_fft_plane_fwd<C, Acc, ONE>, base + 5, p.smem_plane);
+        raise_smem((const void *)k_fft_plane_inv<C, ONE>, base + 6, p.smem_plane);
     }
 }
 
@@ -685,13 +941,13 @@ void fft_plan_build(FftPlan &p, int mixed, cudaStream_t st) {
         FftSysDev &F = p.hsys[s];
         for (int d = 0; d < 3; ++d) {
             fft_passes(F.K[d], F.ax[d]);
+            if (d == 0) fft_passes_reversed(F.K[0], F.ax[0], F.axi);
             if (F.K[d] > p.kmax) p.kmax = F.K[d];
         }
         int nzb = (F.K[0] * F.K[1] + p.zlines - 1) / p.zlines;
         for (int u = 0; u < nzb; ++u) z.push_back({s, u});
-        int chunks = (F.Kh + p.cols - 1) / p.cols;
-        for (int u = 0; u < F.K[0] * chunks; ++u) y.push_back({s, u});
-        for (int u = 0; u < F.K[1] * chunks; ++u) x.push_back({s, u});
+        for (int u = 0; u < (F.K[0] * F.Kh + p.cols - 1) / p.cols; ++u) y.push_back({s, u});
+        for (int u = 0; u < (F.K[1] * F.Kh + p.cols - 1) / p.cols; ++u) x.push_back({s, u});
         for (int u = 0; u < F.K[0]; ++u) pl.push_back({s, u});
         // plane path geometry: whole-plane scratch when it fits
         int ldq = F.K[1] | 1, ldz = F.K[2] | 1;
@@ -704,6 +960,8 @@ void fft_plan_build(FftPlan &p, int mixed, cudaStream_t st) {
     p.smem_z = fft_line_smem(p.zlines / 2, p.kmax, csz);
     p.smem_y = fft_line_smem(p.cols, p.kmax, csz);
     p.smem_x = p.smem_y;
+    p.zthreads = fft_line_threads(p.hsys, 2, p.zlines / 2);
+    p.cthreads = std::max(fft_line_threads(p.hsys, 0, p.cols), fft_line_threads(p.hsys, 1, p.cols));
     // the plane path keeps a plane and two scratch buffers in shared memory;
     // the scratch shrinks to a chunk of lines when the plane is large
     const size_t budget = 200 * 1024 / csz;
@@ -752,10 +1010,11 @@ void fft_plan_build(FftPlan &p, int mixed, cudaStream_t st) {
         std::memcpy(img.data() + bs + bz + by + bx, pl.data(), sizeof(FftWork) * p.npl);
         cudaMemcpyAsync(b, img.data(), need, cudaMemcpyHostToDevice, st);
     }
+    const bool one = p.hsys.size() == 1;
     if (mixed)
-        raise_all<float2, int, float>(p, 0);
+        one ? raise_all<float2, int, float, true>(p, 0) : raise_all<float2, int, float, false>(p, 8);
     else
-        raise_all<double2, double, double>(p, 8);
+        one ? raise_all<double2, double, double, true>(p, 16) : raise_all<double2, double, double, false>(p, 24);
 }
 
 size_t fft_plan_bytes_max(const FftPlan &p) {
@@ -764,10 +1023,10 @@ size_t fft_plan_bytes_max(const FftPlan &p) {
     size_t nz = 0, ny = 0, nx = 0, npl = 0;
     for (int s = 0; s < p.S; ++s) {
         const FftSysDev &F = p.hsys[s];
-        const int Kh = F.K[2] / 2 + 1, chunks = (Kh + 3) / 4;
+        const int Kh = F.K[2] / 2 + 1;
         nz += (F.K[0] * F.K[1] + 7) / 8;
-        ny += (size_t)F.K[0] * chunks;
-        nx += (size_t)F.K[1] * chunks;
+        ny += ((size_t)F.K[0] * Kh + 3) / 4;
+        nx += ((size_t)F.K[1] * Kh + 3) / 4;
         npl += F.K[0];
     }
     return al(sizeof(FftSysDev) * std::max(p.S, 1)) + al(sizeof(FftWork) * (nz + 1)) +

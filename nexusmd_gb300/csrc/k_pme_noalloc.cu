@@ -364,15 +364,18 @@ extern "C" int nxm_pme_reciprocal_noalloc(const double *xyz, const double *charg
         tw += g.K[d];
         fft_passes(g.K[d], F.ax[d]);
     }
+    fft_passes_reversed(g.K[0], F.ax[0], F.axi);
     F.Kh = g.Kh;
     FftPlan plan;  // geometry only; every pointer is into g_pme_scratch
     plan.S = 1;
     plan.zlines = kZLines;
     plan.cols = kCols;
-    int chunks = (g.Kh + kCols - 1) / kCols;
     plan.nz = (g.K[0] * g.K[1] + kZLines - 1) / kZLines;
-    plan.ny = g.K[0] * chunks;
-    plan.nx = g.K[1] * chunks;
+    plan.ny = (g.K[0] * g.Kh + kCols - 1) / kCols;
+    plan.nx = (g.K[1] * g.Kh + kCols - 1) / kCols;
+    plan.hsys.assign(1, F);
+    plan.zthreads = fft_line_threads(plan.hsys, 2, kZLines / 2);
+    plan.cthreads = std::max(fft_line_threads(plan.hsys, 0, kCols), fft_line_threads(plan.hsys, 1, kCols));
     plan.kmax = std::max(g.K[0], std::max(g.K[1], g.K[2]));
     // line path (plan.plane = 0); at most 64 points per axis keeps every
     // block under the 48 KB that needs no shared-memory attribute

@@ -22,6 +22,8 @@ struct FftPasses {
 // Factors n = 2^a 3^b 5^c into passes of radix 10, 9, 8, 6, 4, 2, 3, 5 (the
 // larger first: fewer passes through shared memory).
 void fft_passes(int n, FftPasses &P);
+// The same radices in reverse order.
+void fft_passes_reversed(int n, const FftPasses &P, FftPasses &Q);
 
 // Per-system FFT geometry.  The real grid is row-major K0 x K1 x K2 (z
 // fastest, NonbondedForce.cpp:253); the half spectrum is K0 x K1 x Kh with
@@ -33,6 +35,7 @@ struct FftSysDev {
     long long coff;     // half-spectrum offset (elements)
     int tw[3];          // twiddle-table offset for the length of each axis
     FftPasses ax[3];    // passes per axis
+    FftPasses axi;      // x axis, radices in reverse: the inverse that starts where the forward ends
 };
 
 struct FftWork {
@@ -51,7 +54,8 @@ struct FftPlan {
     size_t ext_cap = 0;
     int nz = 0, ny = 0, nx = 0;
     int zlines = 16;    // real lines per block in the z passes (even)
-    int cols = 8;       // z columns per block in the y and x passes
+    int cols = 8;       // columns per block in the y and x passes (a power of two)
+    int zthreads = 256, cthreads = 256;  // threads per block of the z, and of the y and x passes
     size_t smem_z = 0, smem_y = 0, smem_x = 0;
     int kmax = 0;
     // Plane path: one block per (system, x-plane) runs z then y forward and
@@ -77,5 +81,8 @@ int fft_launch_count(const FftPlan &plan);
 // Shared memory of a line-path block: twiddles and two buffers of `lines`
 // lines of up to kmax complex words.
 size_t fft_line_smem(int lines, int kmax, size_t csz);
+// Threads of a line-path block of `lines` lines along axis d: the butterflies
+// of its largest pass in any system, whole warps, at most 256.
+int fft_line_threads(const std::vector<FftSysDev> &sys, int d, int lines);
 
 }  // namespace nxm
