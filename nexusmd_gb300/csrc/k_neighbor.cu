@@ -339,16 +339,24 @@ void launch_remap_terms(const DevView &v, cudaStream_t st) {
     if (n > 0) k_remap<<<blocks(n, 256), 256, 0, st>>>(v);
 }
 
-void launch_nlist_rebuild(const DevView &v, cudaStream_t st) {
+void launch_nlist_order(const DevView &v, cudaStream_t st) {
     k_assign<<<blocks(v.N, 256), 256, 0, st>>>(v);
     k_scan<<<1, 1024, 0, st>>>(v.flags, v.cell_count, v.cell_start, v.total_cells);
     k_scatter<<<blocks(v.N, 256), 256, 0, st>>>(v);
     k_cellsort<<<blocks(v.total_cells, kSortWarps), kSortWarps * 32, 0, st>>>(v);
     k_permute_gather<<<blocks(v.N, 256), 256, 0, st>>>(v);
     k_permute_scatter<<<blocks(v.N, 256), 256, 0, st>>>(v);
+}
+
+void launch_nlist_lists(const DevView &v, cudaStream_t st) {
     long long nt = (long long)v.nb + v.na + v.nt + v.nex + v.nxc;
     if (nt > 0) k_remap<<<blocks(nt, 256), 256, 0, st>>>(v);
     launch_build(v, st);
+}
+
+void launch_nlist_rebuild(const DevView &v, cudaStream_t st) {
+    launch_nlist_order(v, st);
+    launch_nlist_lists(v, st);
 }
 
 }  // namespace nxm

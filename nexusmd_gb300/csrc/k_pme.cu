@@ -116,8 +116,9 @@ __global__ void __launch_bounds__(256) k_spread(DevView v, const FftSysDev *fs) 
 // one-atom-per-lane; 16 atoms per warp keep twice as many warps in flight as
 // 32 would.  The values are the per-atom kernel's ((q wx) wy) wz, so the
 // grid is identical.
-constexpr int kSpreadWarps = 8, kSpreadAtoms = 16;  // atoms per warp
+constexpr int kSpreadWarps = 8;
 
+template <int kSpreadAtoms>  // atoms per warp
 __global__ void __launch_bounds__(kSpreadWarps * 32) k_spread_warp(DevView v, const FftSysDev *fs) {
     __shared__ float s_w[kSpreadWarps][kSpreadAtoms][16];  // wx[5] wy[5] wz[5] q
     __shared__ int s_i[kSpreadWarps][kSpreadAtoms][4];     // grid index x y z, system (-1: none)
@@ -284,14 +285,25 @@ __global__ void __launch_bounds__(256) k_gather(DevView v, const FftSysDev *fs) 
 // one block per run of cells of a column with its box in shared memory and
 // one thread per atom: 32.8 vs 32.9 us at 94,100 atoms, 112 vs 97 us at
 // 473,400), and five threads per atom (one x-plane each).
-void launch_spread(const DevView &v, const FftPlan &plan, cudaStream_t st) {
-    // the accumulator (int64 fixed point or double, 8 bytes per point) starts at zero
+void launch_clear_grid(const DevView &v, cudaStream_t st) {
+    if (v.N == 0 || !v.grid_acc) return;
     cudaMemsetAsync(v.grid_acc, 0, (v.mixed ? sizeof(int) : sizeof(double)) * (size_t)v.total_grid, st);
+}
+
+// (the accumulator, int32 fixed point or double, starts at zero)
+void launch_spread(const DevView &v, const FftPlan &plan, cudaStream_t st) {
     int t = v.pme_block, nb = (v.N + t - 1) / t;
-    if (v.mixed)
-        k_spread_warp<<<(v.N + kSpreadWarps * kSpreadAtoms - 1) / (kSpreadWarps * kSpreadAtoms), kSpreadWarps * 32, 0,
-                        st>>>(v, plan.dsys);
-    else
+    if (v.mixed) {
+        // 16 atoms per warp, fewer where that leaves SMs idle: a warp takes
+        // its atoms one after the other
+        auto grid = [&](int atoms) { return (v.N + kSpreadWarps * atoms - 1) / (kSpreadWarps * atoms); };
+        if (grid(16) >= 2 * 152)
+            k_spread_warp<16><<<grid(16), kSpreadWarps * 32, 0, st>>>(v, plan.dsys);
+        else if (grid(8) >= 152)
+            k_spread_warp<8><<<grid(8), kSpreadWarps * 32, 0, st>>>(v, plan.dsys);
+        else
+            k_spread_warp<4><<<grid(4), kSpreadWarps * 32, 0, st>>>(v, plan.dsys);
+    } else
         k_spread<double, double><<<nb, t, 0, st>>>(v, plan.dsys);
 }
 
@@ -303,8 +315,9 @@ void launch_gather(const DevView &v, const FftPlan &plan, cudaStream_t st) {
         k_gather<double, double><<<nb, t, 0, st>>>(v, plan.dsys);
 }
 
-void launch_pme(const DevView &v, const FftPlan &plan, int energy, cudaStream_t st) {
+void launch_pme(const DevView &v, const FftPlan &plan, int energy, cudaStream_t st, bool cleared) {
     if (v.N == 0 || plan.nz == 0) return;
+    if (!cleared) launch_clear_grid(v, st);
     launch_spread(v, plan, st);
     launch_fft_convolve(v, plan, energy, st);
     launch_gather(v, plan, st);

@@ -1445,6 +1445,7 @@ std::string Engine::autotune() {
     for (int t : {64, 128, 256}) {
         v_.pme_block = t;
         float ms = time3([&] {
+            launch_clear_grid(v_, st_);
             launch_spread(v_, plan_, st_);
             launch_gather(v_, plan_, st_);
         });
@@ -1518,12 +1519,13 @@ static int force_launch_count(const DevView &v, const FftPlan &plan) {
 // the bonded / pair / exclusion kernels but the force words, which both add
 // to with integer atomics (order-free); the caller joins the streams before
 // the update.
+// (`cleared`: see launch_pme; `pme_done`: the chain was launched before)
 static int force_launches(const DevView &v, const FftPlan &plan, int energy, cudaStream_t st,
-                          cudaStream_t pme_st = nullptr) {
+                          cudaStream_t pme_st = nullptr, bool cleared = false, bool pme_done = false) {
     int n = 0;
     bool nb = (v.force_mask & NXM_FORCE_NONBONDED) != 0;
     if (nb && pme_st) {
-        launch_pme(v, plan, energy, pme_st);
+        if (!pme_done) launch_pme(v, plan, energy, pme_st, cleared);
         n += pme_launch_count(v, plan);
     }
     // bonded terms, exclusion correction and exceptions: one launch
@@ -1578,8 +1580,14 @@ std::string Engine::build_graph_timed(double dt, int report) {
     // head: energy reset and the decision
     e = cudaStreamBeginCaptureToGraph(st_, g, nullptr, nullptr, 0, mode);
     if (e != cudaSuccess) return fail_capture("capture head", e);
+    // (the charge grid is cleared beside the decision)
+    cudaEventRecord(ev_fork_, st_);
+    cudaStreamWaitEvent(st_pme_, ev_fork_, 0);
+    launch_clear_grid(vv, st_pme_);
+    cudaEventRecord(ev_join_, st_pme_);
     if (report) cudaMemsetAsync(vv.E, 0, sizeof(long long) * v_.S * E_SLOTS, st_);
     k_decide_graph<<<1, 1, 0, st_>>>(vv, h);
+    cudaStreamWaitEvent(st_, ev_join_, 0);
     cudaStreamCaptureStatus cs;
     const cudaGraphNode_t *deps = nullptr;
     size_t nd = 0;
@@ -1609,7 +1617,7 @@ std::string Engine::build_graph_timed(double dt, int report) {
     // PME as a parallel branch on the second stream, joined before the update
     cudaEventRecord(ev_fork_, st_);
     cudaStreamWaitEvent(st_pme_, ev_fork_, 0);
-    force_launches(vv, plan_, report ? 1 : 0, st_, st_pme_);
+    force_launches(vv, plan_, report ? 1 : 0, st_, st_pme_, true);
     cudaEventRecord(ev_join_, st_pme_);
     cudaStreamWaitEvent(st_, ev_join_, 0);
     launch_integrate(vv, dt, report >= 2 ? 2 : report, st_);
@@ -1620,6 +1628,26 @@ std::string Engine::build_graph_timed(double dt, int report) {
     G.dt = dt;
     G.ok = true;
     return "";
+}
+
+// A rebuild and all forces, by plain launches.  The PME chain needs the new
+// slot order but none of the lists, so it runs on the second stream beside
+// the list build and the other forces, and joins before what follows.
+int Engine::forced_evaluation(const DevView &vv, int energy) {
+    launch_decide_rebuild(vv, 1, st_);
+    force_rebuild_ = false;
+    launch_nlist_order(vv, st_);
+    const bool pme = (vv.force_mask & NXM_FORCE_NONBONDED) && plan_.nz;
+    if (pme) {
+        cudaEventRecord(ev_fork_, st_);
+        cudaStreamWaitEvent(st_pme_, ev_fork_, 0);
+        launch_pme(vv, plan_, energy, st_pme_);
+        cudaEventRecord(ev_join_, st_pme_);
+    }
+    launch_nlist_lists(vv, st_);
+    const int n = force_launches(vv, plan_, energy, st_, pme ? st_pme_ : nullptr, false, pme);
+    if (pme) cudaStreamWaitEvent(st_, ev_join_, 0);
+    return n;
 }
 
 // One step of report kind `report` (0 none, 1 energies and the x/v/F
@@ -1640,10 +1668,7 @@ std::string Engine::one_step(double dt, int report) {
     }
     const DevView vv = view_for(report);
     if (report) cudaMemsetAsync(vv.E, 0, sizeof(long long) * v_.S * E_SLOTS, st_);
-    launch_decide_rebuild(vv, 1, st_);
-    force_rebuild_ = false;
-    launch_nlist_rebuild(vv, st_);
-    int n = force_launches(vv, plan_, report ? 1 : 0, st_);
+    int n = forced_evaluation(vv, report ? 1 : 0);
     launch_integrate(vv, dt, report >= 2 ? 2 : report, st_);
     launches_per_step_ = n + 2 + launches_per_rebuild_;
     return check("step");
@@ -1790,10 +1815,7 @@ std::string Engine::step(int nsteps, double dt) {
 
 std::string Engine::compute_forces() {
     cudaMemsetAsync(v_.E, 0, sizeof(long long) * v_.S * E_SLOTS, st_);
-    launch_decide_rebuild(v_, 1, st_);
-    force_rebuild_ = false;
-    launch_nlist_rebuild(v_, st_);
-    force_launches(v_, plan_, 1, st_);
+    forced_evaluation(v_, 1);
     launch_export(v_, 1, st_);
     std::string e = check("compute_forces");
     if (!e.empty()) return e;
@@ -1842,6 +1864,7 @@ std::string Engine::profile(int nsteps, double dt, double *ms) {
         if (nb && v_.nex) launch_exclusions(v_, 0, st_);
         if (nb && v_.nxc) launch_exceptions(v_, 0, st_);
         cudaEventRecord(ev[4], st_);
+        if (nb && plan_.nz) launch_clear_grid(v_, st_);
         if (nb && plan_.nz) launch_spread(v_, plan_, st_);
         cudaEventRecord(ev[5], st_);
         if (nb && plan_.nz) launch_fft_convolve(v_, plan_, 0, st_);

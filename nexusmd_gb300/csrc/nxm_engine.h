@@ -175,6 +175,7 @@ private:
     std::string build_graph_timed(double dt, int report);
     void free_graphs();
     std::string one_step(double dt, int report);
+    int forced_evaluation(const DevView &vv, int energy);
     std::string check(const char *what);
     std::string finish_call();
     static void decode_energies(const double *e, const SysHost &H, nxm_energies *out);

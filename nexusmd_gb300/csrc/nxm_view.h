@@ -122,6 +122,10 @@ void launch_exclusions_count(const ExclBuild &b, cudaStream_t st);
 void launch_exclusions_fill(const ExclBuild &b, int *elst, int2 *pairs, cudaStream_t st);
 
 // kernel launchers (one per .cu file group)
+// the rebuild in two parts: the slot order with the per-atom state in it, and
+// what is indexed by it (term indices, lists); launch_nlist_rebuild: both
+void launch_nlist_order(const DevView &v, cudaStream_t st);
+void launch_nlist_lists(const DevView &v, cudaStream_t st);
 void launch_nlist_rebuild(const DevView &v, cudaStream_t st);
 void launch_build(const DevView &v, cudaStream_t st);
 void tiles_set_smem(int hood_cap);
@@ -132,7 +136,10 @@ int launch_bonded(const DevView &v, int energy, cudaStream_t st, int pairs = 0);
 void launch_pairs(const DevView &v, int energy, cudaStream_t st);
 void launch_exclusions(const DevView &v, int energy, cudaStream_t st);
 void launch_exceptions(const DevView &v, int energy, cudaStream_t st);
-void launch_pme(const DevView &v, const struct FftPlan &plan, int energy, cudaStream_t st);
+// PME: spread, transforms and convolution, gather; `cleared`: the charge
+// grid is zero already (launch_clear_grid)
+void launch_pme(const DevView &v, const struct FftPlan &plan, int energy, cudaStream_t st, bool cleared = false);
+void launch_clear_grid(const DevView &v, cudaStream_t st);
 void launch_spread(const DevView &v, const struct FftPlan &plan, cudaStream_t st);
 void launch_fft_convolve(const DevView &v, const struct FftPlan &plan, int energy, cudaStream_t st);
 void launch_gather(const DevView &v, const struct FftPlan &plan, cudaStream_t st);
