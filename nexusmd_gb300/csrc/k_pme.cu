@@ -13,43 +13,13 @@
 #include <algorithm>
 
 #include "nxm_fft.h"
+#include "nxm_spread.cuh"
 #include "nxm_view.h"
 
 namespace nxm {
 
 void launch_fft_convolve(const DevView &v, const FftPlan &p, int energy, cudaStream_t st);
 
-template <typename R>
-__device__ __forceinline__ void bspline5(R dr, R *th, R *dth) {
-    th[4] = 0;
-    th[1] = dr;
-    th[0] = 1 - dr;
-#pragma unroll
-    for (int k = 3; k < 5; k++) {
-        R div = (R)1 / (R)(k - 1);
-        th[k - 1] = div * dr * th[k - 2];
-#pragma unroll
-        for (int l = 1; l < (k - 1); l++)
-            th[k - l - 1] = div * ((dr + l) * th[k - l - 2] + ((R)(k - l) - dr) * th[k - l - 1]);
-        th[0] = div * (1 - dr) * th[0];
-    }
-    dth[0] = -th[0];
-#pragma unroll
-    for (int k = 1; k < 5; k++) dth[k] = th[k - 1] - th[k];
-    R div = (R)0.25;
-    th[4] = div * dr * th[3];
-#pragma unroll
-    for (int l = 1; l < 4; l++) th[4 - l] = div * ((dr + l) * th[3 - l] + ((R)(5 - l) - dr) * th[4 - l]);
-    th[0] = div * (1 - dr) * th[0];
-}
-
-// Mixed-mode grid word: int32 fixed point in units of 2^-24 e, for |Q| <
-// 128 e per point.  A point holds q wx wy wz summed over the atoms whose
-// 5-point stencils cover it, each weight at most 115/192 per axis (< 0.22 per
-// atom), so physical charge densities stay two orders of magnitude inside the
-// range.  Half the bytes of an int64 word per atomic: the spread's L2 atomic
-// traffic is its bound (38 -> 33 us at 94,100 atoms on a 100^3 grid).
-__device__ __forceinline__ int to_grid_fixed(float v) { return __float2int_rn(v * 16777216.0f); }
 __device__ __forceinline__ void grid_add(int *g, float v) { atomicAdd(g, to_grid_fixed(v)); }
 __device__ __forceinline__ void grid_add(double *g, double v) { atomicAdd(g, v); }
 
@@ -167,7 +137,6 @@ __global__ void __launch_bounds__(kSpreadWarps * 32) k_spread_warp(DevView v, co
         s_i[warp][lane][3] = sys;
     }
     __syncwarp();
-    const unsigned full = 0xffffffffu;
     for (int a = 0; a < kSpreadAtoms; ++a) {
         const int sys = s_i[warp][a][3];
         if (sys < 0) continue;
@@ -175,30 +144,7 @@ __global__ void __launch_bounds__(kSpreadWarps * 32) k_spread_warp(DevView v, co
         const int K0 = F.K[0], K1 = F.K[1], K2 = F.K[2];
         int *g = static_cast<int *>(v.grid_acc) + F.roff;
         const float *w = s_w[warp][a];
-        // lane r < 25: grid row (ix, iy) = (r / 5, r % 5) of the atom, its
-        // offset and its weight (q wx) wy
-        long long row_off = 0;
-        float row_w = 0.f;
-        if (lane < 25) {
-            const int ix = lane / 5, iy = lane - 5 * ix;
-            int xi = s_i[warp][a][0] + ix, yi = s_i[warp][a][1] + iy;
-            xi -= xi >= K0 ? K0 : 0;
-            yi -= yi >= K1 ? K1 : 0;
-            row_off = ((long long)xi * K1 + yi) * K2;
-            row_w = w[15] * w[ix] * w[5 + iy];
-        }
-        const int z0 = s_i[warp][a][2];
-        // point p = 5 row + iz: 32 consecutive points per instruction
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int p = lane + 32 * k;
-            const int row = min(p / 5, 24), iz = min(p - 5 * row, 4);  // (clamped past point 124)
-            const long long off = __shfl_sync(full, row_off, row);
-            const float rw = __shfl_sync(full, row_w, row);
-            int zi = z0 + iz;
-            zi -= zi >= K2 ? K2 : 0;
-            if (p < 125) atomicAdd(g + off + zi, to_grid_fixed(rw * w[10 + iz]));
-        }
+        spread_points(w, s_i[warp][a], K0, K1, K2, g, lane);
     }
 }
 

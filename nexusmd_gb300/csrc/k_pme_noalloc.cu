@@ -1,7 +1,6 @@
 // Reciprocal-space PME on caller-owned device buffers that allocates nothing:
 // every intermediate (fixed-point charge grid, half spectrum, real grid,
-// influence function, B-spline moduli, FFT twiddles and work lists, energy
-// word) lives in one file-scope device array of fixed size, g_pme_scratch.
+// influence function, per-axis tables, FFT twiddles, energy word) lives in one file-scope device array of fixed size, g_pme_scratch.
 //
 // The arithmetic is the engine's mixed-precision PME step (k_pme.cu spread
 // and gather, k_fft.cu transforms, the influence function of nxm_engine.cu),
@@ -35,6 +34,7 @@
 
 #include "../../include/nxm.h"
 #include "nxm_fft.h"
+#include "nxm_spread.cuh"
 #include "nxm_view.h"
 
 namespace nxm {
@@ -49,17 +49,13 @@ constexpr int kStaticMaxK = 64;
 constexpr int kStaticMaxKh = kStaticMaxK / 2 + 1;
 constexpr int kZLines = 16;  // real lines per block in the z passes
 constexpr int kCols = 8;     // columns per block in the y and x passes
-constexpr int kMaxWork = kStaticMaxK * ((kStaticMaxKh + kCols - 1) / kCols);  // >= every work list
-
 constexpr size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // byte offsets of the regions of g_pme_scratch
 constexpr size_t kOffE = 0;                                                   // long long[E_SLOTS]
-constexpr size_t kOffSys = kOffE + align256(sizeof(long long) * E_SLOTS);     // FftSysDev
-constexpr size_t kOffWork = kOffSys + align256(sizeof(FftSysDev));            // 3 x FftWork[kMaxWork]
-constexpr size_t kOffTw = kOffWork + align256(3 * sizeof(FftWork) * kMaxWork);  // float2[3][K]
-constexpr size_t kOffMod = kOffTw + align256(sizeof(float2) * 3 * kStaticMaxK);  // double[3][K]
-constexpr size_t kOffAcc = kOffMod + align256(sizeof(double) * 3 * kStaticMaxK);
+constexpr size_t kOffTw = kOffE + align256(sizeof(long long) * E_SLOTS);      // float2[3][K]
+constexpr size_t kOffAxis = kOffTw + align256(sizeof(float2) * 3 * kStaticMaxK);  // double2[3][K]
+constexpr size_t kOffAcc = kOffAxis + align256(sizeof(double2) * 3 * kStaticMaxK);
 constexpr size_t kGridPts = (size_t)kStaticMaxK * kStaticMaxK * kStaticMaxK;
 constexpr size_t kSpecPts = (size_t)kStaticMaxK * kStaticMaxK * kStaticMaxKh;
 constexpr size_t kOffReal = kOffAcc + align256(sizeof(int) * kGridPts);
@@ -85,31 +81,6 @@ __device__ __forceinline__ T *region(unsigned char *base, size_t off) {
     return reinterpret_cast<T *>(base + off);
 }
 
-// B-spline weights and derivatives of order 5 at fraction dr, in the
-// operation order of computeBSplineParameters (NonbondedForce.cpp:144-182).
-__device__ __forceinline__ void spline5(float dr, float *th, float *dth) {
-    th[4] = 0.f;
-    th[1] = dr;
-    th[0] = 1.f - dr;
-#pragma unroll
-    for (int k = 3; k < 5; k++) {
-        float div = 1.f / (float)(k - 1);
-        th[k - 1] = div * dr * th[k - 2];
-#pragma unroll
-        for (int l = 1; l < (k - 1); l++)
-            th[k - l - 1] = div * ((dr + l) * th[k - l - 2] + ((float)(k - l) - dr) * th[k - l - 1]);
-        th[0] = div * (1.f - dr) * th[0];
-    }
-    dth[0] = -th[0];
-#pragma unroll
-    for (int k = 1; k < 5; k++) dth[k] = th[k - 1] - th[k];
-    float div = 0.25f;
-    th[4] = div * dr * th[3];
-#pragma unroll
-    for (int l = 1; l < 4; l++) th[4 - l] = div * ((dr + l) * th[3 - l] + ((float)(5 - l) - dr) * th[4 - l]);
-    th[0] = div * (1.f - dr) * th[0];
-}
-
 // Grid base index and fraction of one coordinate (NonbondedForce.cpp:51-71:
 // the grid is anchored at the origin).
 __device__ __forceinline__ void grid_coord(double p, double invL, int K, int &idx, float &fr) {
@@ -120,142 +91,114 @@ __device__ __forceinline__ void grid_coord(double p, double invL, int K, int &id
     idx = ti % K;
 }
 
-// ---- set-up: clear the accumulator and the energy word, write the FFT
-// geometry, work lists and twiddles; block 0 also computes the B-spline
-// moduli |b(k)|^2 of the three axes with the neighbour average for values
-// below 1e-7 (NonbondedForce.cpp:75-142).
-__global__ void k_noalloc_setup(unsigned char *scr, FftSysDev F, int nz, int ny, int nx) {
-    __shared__ double s_mod[3][kStaticMaxK];
-    int *acc = region<int>(scr, kOffAcc);
-    long long npts = (long long)F.K[0] * F.K[1] * F.K[2];
-    long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    long long nthr = (long long)gridDim.x * blockDim.x;
-    for (long long i = tid; i < npts; i += nthr) acc[i] = 0;
-    if (tid < E_SLOTS) region<long long>(scr, kOffE)[tid] = 0;
-    if (tid == 0) *region<FftSysDev>(scr, kOffSys) = F;
-    FftWork *zw = region<FftWork>(scr, kOffWork);
-    FftWork *yw = zw + kMaxWork, *xw = yw + kMaxWork;
-    for (long long i = tid; i < kMaxWork; i += nthr) {
-        int u = (int)i;
-        if (u < nz) zw[u] = FftWork{0, u};
-        if (u < ny) yw[u] = FftWork{0, u};
-        if (u < nx) xw[u] = FftWork{0, u};
+// |b(k)|^2 of one axis: the order-5 spline's values at the integers are
+// 1/24, 11/24, 11/24, 1/24, so with c = cos(2 pi k / K) the sum
+// |1/24 (z + z^4) + 11/24 (z^2 + z^3)|^2 is 2 (1 + c) (11/24 + (2c - 1)/24)^2
+// (NonbondedForce.cpp:75-142 sums sines and cosines: ten times the FP64 work).
+__device__ __forceinline__ double modulus2(int k, int K) {
+    const double c = cospi(2.0 * (double)k / (double)K);
+    const double t = (10.0 + 2.0 * c) * (1.0 / 24.0);
+    return 2.0 * (1.0 + c) * t * t;
+}
+
+// ---- set-up, blocks of one warp's worth of FP64 work each (the pipe is
+// narrow): the first kAxisBlocks blocks make the per-axis tables -- twiddles,
+// and (m_d^2, exp(-pi^2 m_d^2 / alpha^2) / |b|^2) -- one entry per lane, with
+// the neighbour average for |b|^2 below 1e-7; the others clear the
+// accumulator and the energy words.  The axis tables replace an exponential
+// and a modulus sum per spectrum element and a serial block of sines and
+// cosines: 24,000 atoms on 64^3, the whole entry 130 -> 77 us.
+constexpr int kAxisBlocks = 3 * kStaticMaxK / 32;
+
+__global__ void __launch_bounds__(256) k_noalloc_setup(unsigned char *scr, Geometry g) {
+    if (blockIdx.x >= kAxisBlocks) {
+        int4 *acc = region<int4>(scr, kOffAcc);
+        const int n = (g.K[0] * g.K[1] * g.K[2] + 3) / 4;  // (the region holds whole int4)
+        const int t0 = (blockIdx.x - kAxisBlocks) * blockDim.x + threadIdx.x, nt = (gridDim.x - kAxisBlocks) * blockDim.x;
+        for (int i = t0; i < n; i += nt) acc[i] = make_int4(0, 0, 0, 0);
+        if (t0 < E_SLOTS) region<long long>(scr, kOffE)[t0] = 0;
+        return;
     }
-    float2 *tw = region<float2>(scr, kOffTw);
-    for (long long i = tid; i < F.K[0] + F.K[1] + F.K[2]; i += nthr) {
-        int d = i < F.K[0] ? 0 : (i < F.K[0] + F.K[1] ? 1 : 2);
-        int t = (int)i - F.tw[d];
-        double a = -2.0 * kPi * (double)t / (double)F.K[d];
+    if (threadIdx.x >= 32) return;
+    const int d = blockIdx.x / (kStaticMaxK / 32), k = (blockIdx.x % (kStaticMaxK / 32)) * 32 + threadIdx.x;
+    const int K = g.K[d];
+    if (k >= K) return;
+    {
         double s, c;
-        sincos(a, &s, &c);
-        tw[i] = make_float2((float)c, (float)s);
+        sincospi(-2.0 * (double)k / (double)K, &s, &c);
+        region<float2>(scr, kOffTw)[(d > 0 ? g.K[0] : 0) + (d > 1 ? g.K[1] : 0) + k] = make_float2((float)c, (float)s);
     }
-    if (blockIdx.x != 0) return;
-    // spline values at the integer points, computed as the reference does
-    double data[kOrder] = {0, 0, 0, 0, 0};
-    data[0] = 1.0;
-    for (int i = 3; i < kOrder; i++) {
-        double div = 1.0 / (i - 1);
-        data[i - 1] = 0.0;
-        for (int j = 1; j < (i - 1); j++) data[i - j - 1] = div * (j * data[i - j - 2] + (i - j) * data[i - j - 1]);
-        data[0] = div * data[0];
-    }
-    double div = 1.0 / (kOrder - 1);
-    data[kOrder - 1] = div * data[kOrder - 2];
-    for (int i = 1; i < (kOrder - 1); i++)
-        data[kOrder - i - 1] = div * (i * data[kOrder - i - 2] + (kOrder - i) * data[kOrder - i - 1]);
-    data[0] = div * data[0];
-    for (int e = threadIdx.x; e < F.K[0] + F.K[1] + F.K[2]; e += blockDim.x) {
-        int d = e < F.K[0] ? 0 : (e < F.K[0] + F.K[1] ? 1 : 2);
-        int K = F.K[d], i = e - F.tw[d];
-        double sc = 0.0, ss = 0.0;
-        // b[j] = data[j - 1] for j = 1..order, zero elsewhere
-        for (int j = 1; j <= kOrder && j < K; ++j) {
-            double arg = (2 * kPi * i * j) / K;
-            sc += data[j - 1] * cos(arg);
-            ss += data[j - 1] * sin(arg);
-        }
-        s_mod[d][i] = sc * sc + ss * ss;
-    }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        int d = threadIdx.x, K = F.K[d];
-        double *m = s_mod[d];
-        for (int i = 0; i < K; i++)
-            if (m[i] < 1e-7) m[i] = (m[(i - 1 + K) % K] + m[(i + 1) % K]) / 2.0;
-        double *out = region<double>(scr, kOffMod) + d * kStaticMaxK;
-        for (int i = 0; i < K; i++) out[i] = m[i];
-    }
+    double mod = modulus2(k, K);
+    if (mod < 1e-7) mod = (modulus2((k - 1 + K) % K, K) + modulus2((k + 1) % K, K)) / 2.0;
+    const double mh = (k < (K + 1) / 2 ? k : k - K) * g.invL[d];
+    const double m2 = mh * mh;
+    region<double2>(scr, kOffAxis)[d * kStaticMaxK + k] =
+        make_double2(m2, exp(-(kPi * kPi / (g.alpha * g.alpha)) * m2) / mod);
 }
 
-// ---- influence function on the half spectrum (NonbondedForce.cpp:323-388).
-__global__ void k_noalloc_eterm(unsigned char *scr, Geometry g) {
-    const double *mod = region<double>(scr, kOffMod);
-    float *et = region<float>(scr, kOffEterm);
-    int K0 = g.K[0], K1 = g.K[1], K2 = g.K[2], Kh = g.Kh;
-    long long n = (long long)K0 * K1 * Kh;
-    double factor = kPi * kPi / (g.alpha * g.alpha);
-    double boxfactor = kPi * g.L[0] * g.L[1] * g.L[2];
-    int maxkx = (K0 + 1) / 2, maxky = (K1 + 1) / 2, maxkz = (K2 + 1) / 2;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        int kz = (int)(i % Kh);
-        long long r = i / Kh;
-        int ky = (int)(r % K1), kx = (int)(r / K1);
-        if (i == 0) {
-            et[0] = 0.f;
-            continue;
-        }
-        double mhx = ((kx < maxkx) ? kx : (kx - K0)) * (1 / g.L[0]);
-        double mhy = ((ky < maxky) ? ky : (ky - K1)) * (1 / g.L[1]);
-        double mhz = ((kz < maxkz) ? kz : (kz - K2)) * (1 / g.L[2]);
-        double m2 = __dadd_rn(__dadd_rn(__dmul_rn(mhx, mhx), __dmul_rn(mhy, mhy)), __dmul_rn(mhz, mhz));
-        double bx = boxfactor * mod[kx];
-        double denom = m2 * bx * mod[kStaticMaxK + ky] * mod[2 * kStaticMaxK + kz];
-        et[i] = (float)(kOne4PiEps0 * exp(-factor * m2) / denom);
-    }
+// 1 / x to 2^-50 from the FP32 reciprocal and two Newton steps (an FP64
+// division takes three times the FP64 instructions).
+__device__ __forceinline__ double reciprocal(double x) {
+    if (!(x > 1e-30 && x < 1e30)) return 1.0 / x;
+    double r = (double)fast_rcp((float)x);
+    r = fma(r, fma(-x, r, 1.0), r);
+    return fma(r, fma(-x, r, 1.0), r);
 }
 
-// ---- spread: one thread per atom, int32 fixed-point grid (2^-24 e units,
-// the grid word the FFT's first pass reads).
-__global__ void __launch_bounds__(128) k_noalloc_spread(unsigned char *scr, Geometry g, const double *xyz,
-                                                        const double *charge, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int idx[3];
-    float fr[3], th[3][5], dth[3][5];
+// ---- spread (the first nspread blocks; a warp takes kAtoms atoms one after
+// the other, as the engine's k_spread_warp: int32 fixed point, 2^-24 e, the
+// grid word the FFT's first pass reads) and, in the blocks behind, the
+// influence function on the half spectrum (NonbondedForce.cpp:323-388), which
+// needs the axis tables only: one launch for the two.
+constexpr int kAtoms = 8, kSpreadBlockWarps = 4;
+
+__global__ void __launch_bounds__(kSpreadBlockWarps * 32) k_noalloc_spread(unsigned char *scr, Geometry g,
+                                                                           const double *xyz, const double *charge,
+                                                                           int n, int nspread) {
+    if ((int)blockIdx.x >= nspread) {
+        const double2 *ax = region<double2>(scr, kOffAxis), *ay = ax + kStaticMaxK, *az = ay + kStaticMaxK;
+        float *et = region<float>(scr, kOffEterm);
+        const int K1 = g.K[1], Kh = g.Kh, total = g.K[0] * K1 * Kh;
+        const double f = kOne4PiEps0 / (kPi * g.L[0] * g.L[1] * g.L[2]);
+        for (int i = (blockIdx.x - nspread) * blockDim.x + threadIdx.x; i < total;
+             i += (gridDim.x - nspread) * blockDim.x) {
+            const int r = i / Kh, kz = i - r * Kh, kx = r / K1, ky = r - kx * K1;
+            const double2 x = ax[kx], y = ay[ky], z = az[kz];
+            et[i] = i == 0 ? 0.f : (float)(f * x.y * y.y * z.y * reciprocal(x.x + y.x + z.x));
+        }
+        return;
+    }
+    __shared__ float s_w[kSpreadBlockWarps][kAtoms][16];  // wx[5] wy[5] wz[5] q
+    __shared__ int s_i[kSpreadBlockWarps][kAtoms][3];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int first = (blockIdx.x * kSpreadBlockWarps + warp) * kAtoms;
+    // lane 3 a + d prepares axis d of atom a
+    if (lane < 3 * kAtoms && first + lane / 3 < n) {
+        const int a = lane / 3, d = lane - 3 * a;
+        const size_t i = (size_t)first + a;
+        int idx;
+        float fr, th[5], dth[5];
+        grid_coord(xyz[3 * i + d], g.invL[d], g.K[d], idx, fr);
+        bspline5<float>(fr, th, dth);
+        s_i[warp][a][d] = idx;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        grid_coord(xyz[3 * (size_t)i + d], g.invL[d], g.K[d], idx[d], fr[d]);
-        spline5(fr[d], th[d], dth[d]);
+        for (int k = 0; k < 5; ++k) s_w[warp][a][5 * d + k] = th[k];
+        if (d == 0) s_w[warp][a][15] = (float)charge[i];
     }
-    float q = (float)charge[i];
+    __syncwarp();
     int *acc = region<int>(scr, kOffAcc);
-    int K0 = g.K[0], K1 = g.K[1], K2 = g.K[2];
-    for (int ix = 0; ix < 5; ++ix) {
-        int xi = idx[0] + ix;
-        xi -= xi >= K0 ? K0 : 0;
-        float qx = q * th[0][ix];
-        for (int iy = 0; iy < 5; ++iy) {
-            int yi = idx[1] + iy;
-            yi -= yi >= K1 ? K1 : 0;
-            float qxy = qx * th[1][iy];
-            long long row = ((long long)xi * K1 + yi) * K2;
-#pragma unroll
-            for (int iz = 0; iz < 5; ++iz) {
-                int zi = idx[2] + iz;
-                zi -= zi >= K2 ? K2 : 0;
-                atomicAdd(acc + row + zi, __float2int_rn(qxy * th[2][iz] * 16777216.0f));
-            }
-        }
-    }
+    for (int a = 0; a < min(kAtoms, n - first); ++a)
+        spread_points(s_w[warp][a], s_i[warp][a], g.K[0], g.K[1], g.K[2], acc, lane);
 }
 
-// ---- gather: one thread per atom; writes the force (kJ/mol/nm) and, from
-// thread 0, the reciprocal energy.
-__global__ void __launch_bounds__(128) k_noalloc_gather(unsigned char *scr, Geometry g, const double *xyz,
-                                                        const double *charge, int n, double *force,
-                                                        double *energy) {
+// ---- gather: one thread per atom, the stencil row by row (the z sums first,
+// then the row's x/y weights); writes the force (kJ/mol/nm) and, from thread
+// 0, the reciprocal energy.
+constexpr int kGatherThreads = 64;
+
+__global__ void __launch_bounds__(kGatherThreads) k_noalloc_gather(unsigned char *scr, Geometry g, const double *xyz,
+                                                                   const double *charge, int n, double *force,
+                                                                   double *energy) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) *energy = (double)region<long long>(scr, kOffE)[E_RECIP] * kEnergyUnscale;
     if (i >= n) return;
@@ -264,30 +207,36 @@ __global__ void __launch_bounds__(128) k_noalloc_gather(unsigned char *scr, Geom
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         grid_coord(xyz[3 * (size_t)i + d], g.invL[d], g.K[d], idx[d], fr[d]);
-        spline5(fr[d], th[d], dth[d]);
+        bspline5<float>(fr[d], th[d], dth[d]);
     }
     const float *grid = region<float>(scr, kOffReal);
-    int K0 = g.K[0], K1 = g.K[1], K2 = g.K[2];
+    const int K0 = g.K[0], K1 = g.K[1], K2 = g.K[2];
+    int zo[5];
+#pragma unroll
+    for (int iz = 0; iz < 5; ++iz) {
+        const int zi = idx[2] + iz;
+        zo[iz] = zi >= K2 ? zi - K2 : zi;
+    }
     float fx = 0.f, fy = 0.f, fz = 0.f;
+#pragma unroll
     for (int ix = 0; ix < 5; ++ix) {
         int xi = idx[0] + ix;
         xi -= xi >= K0 ? K0 : 0;
+#pragma unroll
         for (int iy = 0; iy < 5; ++iy) {
             int yi = idx[1] + iy;
             yi -= yi >= K1 ? K1 : 0;
-            const float *row = grid + ((long long)xi * K1 + yi) * K2;
-            float txy = th[0][ix] * th[1][iy];
-            float dxy = dth[0][ix] * th[1][iy];
-            float tdy = th[0][ix] * dth[1][iy];
+            const float *row = grid + (xi * K1 + yi) * K2;
+            float sz = 0.f, sdz = 0.f;
 #pragma unroll
             for (int iz = 0; iz < 5; ++iz) {
-                int zi = idx[2] + iz;
-                zi -= zi >= K2 ? K2 : 0;
-                float gv = row[zi];
-                fx += dxy * th[2][iz] * gv;
-                fy += tdy * th[2][iz] * gv;
-                fz += txy * dth[2][iz] * gv;
+                const float gv = row[zo[iz]];
+                sz = fmaf(th[2][iz], gv, sz);
+                sdz = fmaf(dth[2][iz], gv, sdz);
             }
+            fx = fmaf(dth[0][ix] * th[1][iy], sz, fx);
+            fy = fmaf(th[0][ix] * dth[1][iy], sz, fy);
+            fz = fmaf(th[0][ix] * th[1][iy], sdz, fz);
         }
     }
     float q = (float)charge[i];
@@ -382,11 +331,6 @@ extern "C" int nxm_pme_reciprocal_noalloc(const double *xyz, const double *charg
     plan.smem_z = fft_line_smem(kZLines / 2, plan.kmax, sizeof(float2));
     plan.smem_y = fft_line_smem(kCols, plan.kmax, sizeof(float2));
     plan.smem_x = plan.smem_y;
-    plan.dsys = reinterpret_cast<FftSysDev *>(scr + kOffSys);
-    plan.zwork = reinterpret_cast<FftWork *>(scr + kOffWork);
-    plan.ywork = plan.zwork + kMaxWork;
-    plan.xwork = plan.ywork + kMaxWork;
-
     DevView v{};
     v.N = n_atoms;
     v.S = 1;
@@ -407,12 +351,13 @@ extern "C" int nxm_pme_reciprocal_noalloc(const double *xyz, const double *charg
     if (pending != cudaSuccess)
         return fail(NXM_ERR_CUDA, std::string(fn) + "a CUDA error was already pending: " +
                                       cudaGetErrorString(pending));
-    k_noalloc_setup<<<152, 256, 0, st>>>(scr, F, plan.nz, plan.ny, plan.nx);
-    k_noalloc_eterm<<<(int)std::min<long long>((v.total_cgrid + 255) / 256, 1216), 256, 0, st>>>(scr, g);
-    if (n_atoms > 0) k_noalloc_spread<<<(n_atoms + 127) / 128, 128, 0, st>>>(scr, g, xyz, charge, n_atoms);
+    k_noalloc_setup<<<kAxisBlocks + 152, 256, 0, st>>>(scr, g);
+    const int nspread = (n_atoms + kSpreadBlockWarps * kAtoms - 1) / (kSpreadBlockWarps * kAtoms);
+    const int neterm = (int)std::min<long long>((v.total_cgrid + kSpreadBlockWarps * 32 - 1) / (kSpreadBlockWarps * 32), 608);
+    k_noalloc_spread<<<nspread + neterm, kSpreadBlockWarps * 32, 0, st>>>(scr, g, xyz, charge, n_atoms, nspread);
     launch_fft_convolve(v, plan, 1, st);
-    k_noalloc_gather<<<std::max(1, (n_atoms + 127) / 128), 128, 0, st>>>(scr, g, xyz, charge, n_atoms, force,
-                                                                          energy);
+    k_noalloc_gather<<<std::max(1, (n_atoms + kGatherThreads - 1) / kGatherThreads), kGatherThreads, 0, st>>>(
+        scr, g, xyz, charge, n_atoms, force, energy);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(NXM_ERR_CUDA, std::string(fn) + "launch failed: " + cudaGetErrorString(e));
     return NXM_OK;
