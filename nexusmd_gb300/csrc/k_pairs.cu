@@ -137,6 +137,11 @@ __device__ __forceinline__ float2 lds64(unsigned a) {
     asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
     return v;
 }
+// The value in a register: not worked out again where it is used.
+__device__ __forceinline__ unsigned held(unsigned a) {
+    asm volatile("mov.u32 %0, %0;" : "+r"(a));
+    return a;
+}
 __device__ __forceinline__ int lds32(unsigned a) {
     int v;
     asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a));
@@ -189,7 +194,9 @@ struct BuildAtom {
     }
     __device__ __forceinline__ bool excluded(const DevView &v, int oj) const {
         bool ex = oj == oi;
+#pragma unroll 1
         for (int e = 0; e < min(ne, 32); ++e) ex |= lds32(list + 4 * e) == oj;
+#pragma unroll 1
         for (int e = 32; e < ne; ++e) ex |= v.excl_lst[e0 + e] == oj;
         return ex;
     }
@@ -210,8 +217,9 @@ struct BuildAtom {
 // Bound by instruction issue: a warp tests 32 candidates against both atoms
 // with one load of each candidate and one compaction, so an atom costs about
 // two thirds of what a list of its own does, and half the list traffic.
-// 94,100 atoms: 312 us with a list per atom, 241 so (257 -> 179 M warp
-// instructions); 473,400: 1,730 -> 1,330.
+// 94,100 atoms: 312 us with a list per atom, 221 so (257 -> 167 M warp
+// instructions).  Its loops are kept rolled: unrolled by the compiler they
+// spend more on moving registers than the unrolling saves (241 -> 221 us).
 //
 // W warps per block: 16 (two blocks per SM) or, when two blocks' shared
 // memory does not fit on an SM, 32 (one block per SM, the same 32 warps).
@@ -263,8 +271,8 @@ __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_build(DevVi
     const float csx = (float)S.cs[0], csy = (float)S.cs[1], csz = (float)S.cs[2], icsz = 1.0f / csz;
     int g = G.ncell;
     uint16_t *buf = s_buf + warp * kBuildWarpWords, *keep = buf + 512;
-    const unsigned q_addr = smem_addr(s_q), buf_addr = smem_addr(buf), keep_addr = smem_addr(keep),
-                   ex_addr = keep_addr + 2 * kKeep, lt = (1u << lane) - 1u;
+    const unsigned keep_addr = smem_addr(keep), ex_addr = keep_addr + 2 * kKeep, lt = (1u << lane) - 1u;
+    const unsigned tile_lane = held(smem_addr(s_q) + 16 * lane), buf_addr = held(smem_addr(buf));
     const int cap_entries = pair_stride(v.stride);
     for (int q = q0 + warp; q < q1; q += nw) {
         const int2 ab = v.ipair[q];
@@ -306,6 +314,7 @@ __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_build(DevVi
                     // first such atom lies in cell zlo and the last in cell
                     // zhi, so each search covers one cell.
                     int l = b[zlo + 2], r = b[zlo + 3];
+#pragma unroll 1
                     while (l < r) {
                         int mid = (l + r) >> 1;
                         if (s_q[mid].z < zl)
@@ -316,6 +325,7 @@ __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_build(DevVi
                     kb = l;
                     l = max(b[zhi + 2], kb);
                     r = b[zhi + 3];
+#pragma unroll 1
                     while (l < r) {
                         int mid = (l + r) >> 1;
                         if (s_q[mid].z <= zh)
@@ -350,19 +360,26 @@ __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_build(DevVi
             count = newc;
         };
         unsigned rows = __ballot_sync(full, ke > kb);
+#pragma unroll 1
         while (rows) {
             int r = __ffs(rows) - 1;
             rows &= rows - 1;
             const int rb = __shfl_sync(full, kb, r), re = __shfl_sync(full, ke, r);
-            for (int k = rb + lane; k - lane < re; k += 32) {
-                // k past the row's end reads a later row or the chunk
+            unsigned at = tile_lane + 16 * rb;
+            int entry0 = (rb + lane) << kEntryShift;
+#pragma unroll 1
+            for (int left = re - rb; left > 0; left -= 32, at += 512, entry0 += 32 << kEntryShift) {
+                // a place past the row's end reads a later row or the chunk
                 // buffers behind the tile, inside the block's shared
                 // memory; such a lane is no candidate
-                const float4 c = lds128(q_addr + 16 * k);
-                const bool in_row = k < re;
-                bool inA = in_row & (A.r2(c) < rl2), inB = in_row & (B.r2(c) < rl2);
+                const float4 c = lds128(at);
+                const float reach = lane < left ? rl2 : -1.0f;
+                const float2 dx = make_float2(A.x - c.x, B.x - c.x), dy = make_float2(A.y - c.y, B.y - c.y),
+                             dz = make_float2(A.z - c.z, B.z - c.z);
+                const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+                bool inA = r2.x < reach, inB = r2.y < reach;
                 const int oj = __float_as_int(c.w);
-                int entry = k << kEntryShift;
+                int entry = entry0;
                 bool cand = inA | inB;
                 if (__any_sync(full, cand && ((unsigned)(oj - A.lo) <= A.win || (unsigned)(oj - B.lo) <= B.win))) {
                     const bool exA = A.excluded(v, oj), exB = B.excluded(v, oj);
@@ -393,6 +410,7 @@ __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_build(DevVi
             }
         }
         __syncwarp();
+#pragma unroll 1
         for (int t0 = 0; t0 < kept; t0 += 32) {
             flagged |= 1u << (count >> 8) | 1u << min((count + 31) >> 8, 31);
             append(t0 + lane < kept, keep[min(t0 + lane, kKeep - 1)]);
@@ -410,9 +428,11 @@ __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_build(DevVi
             // The capacity is an atom's: its own entries, whatever the
             // union's count.  Counted apart, as it is hardly ever asked.
             int nA = 0, nB = 0;
+#pragma unroll 1
             for (unsigned left = __ballot_sync(full, ke > kb); left; left &= left - 1) {
                 const int r = __ffs(left) - 1;
                 const int rb = __shfl_sync(full, kb, r), re = __shfl_sync(full, ke, r);
+#pragma unroll 1
                 for (int k = rb + lane; k < re; k += 32) {
                     const float4 c = s_q[k];
                     const int oj = __float_as_int(c.w);
