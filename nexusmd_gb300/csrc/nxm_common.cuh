@@ -271,6 +271,8 @@ __device__ __forceinline__ long long energy_fixed(float v) {
 // one system (per lane otherwise).
 __device__ __forceinline__ void energy_add_f(long long *E, int sys, int term, float v) {
     const unsigned full = 0xffffffffu;
+    // (a warp of the per-term kernel holds one or two kinds of terms)
+    if (!__any_sync(full, v != 0.0f)) return;
     long long w = energy_fixed(v);
     const int s0 = __shfl_sync(full, sys, 0);
     if (__all_sync(full, sys == s0)) {
