@@ -180,6 +180,28 @@ __global__ void k_export(DevView v, int with_forces) {
     }
 }
 
+// Positions and velocities in original atom order, x y z per atom, into x and
+// v (either may be null).
+__global__ void k_state_out(DevView v, double *x, double *vel) {
+    int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= v.N) return;
+    const size_t o = 3 * (size_t)v.orig[s];
+    if (x) {
+        x[o] = v.x[s];
+        x[o + 1] = v.y[s];
+        x[o + 2] = v.z[s];
+    }
+    if (vel) {
+        vel[o] = v.vx[s];
+        vel[o + 1] = v.vy[s];
+        vel[o + 2] = v.vz[s];
+    }
+}
+
+void launch_state_out(const DevView &v, double *x, double *vel, cudaStream_t st) {
+    if (v.N) k_state_out<<<(v.N + 255) / 256, 256, 0, st>>>(v, x, vel);
+}
+
 void launch_integrate(const DevView &v, double dt, int report, cudaStream_t st) {
     int nb = (v.N + 255) / 256;
     if (v.mixed)

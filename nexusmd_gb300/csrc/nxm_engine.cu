@@ -7,6 +7,8 @@
 // The step is the reference's CalculateForces -> Report -> Integrate
 // (core/baseline/src/Engine.cpp:162-188) as a fixed sequence of kernel
 // launches on one stream, everything resident on the device.
+#include <unistd.h>
+
 #include <algorithm>
 #include <chrono>
 #include <cstdlib>
@@ -433,6 +435,17 @@ static void *pinned_alloc(size_t b) {
         return nullptr;
     }
     return p;
+}
+
+// Writes to every page of an output array that a device copy is about to
+// fill: pages the process has not touched yet are mapped by the host here
+// (while the device works), which is far cheaper than by the copy faulting
+// them in (8.6 MB of fresh pages: 9 ms).
+static void touch_pages(void *p, size_t bytes) {
+    static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    volatile char *c = static_cast<volatile char *>(p);
+    for (size_t k = 0; k < bytes; k += page) c[k] = 0;
+    if (bytes) c[bytes - 1] = 0;
 }
 
 static void pinned_free(void *p) {
@@ -1887,8 +1900,11 @@ std::string Engine::profile(int nsteps, double dt, double *ms) {
 }
 
 std::string Engine::get_snapshot(double *x, double *v, double *f) {
-    cudaStreamSynchronize(st_);
     size_t b = sizeof(double) * 3 * (size_t)N_;
+    if (x) touch_pages(x, b);
+    if (v) touch_pages(v, b);
+    if (f) touch_pages(f, b);
+    cudaStreamSynchronize(st_);
     if (x) cudaMemcpy(x, v_.snap_x, b, cudaMemcpyDeviceToHost);
     if (v) cudaMemcpy(v, v_.snap_v, b, cudaMemcpyDeviceToHost);
     if (f) cudaMemcpy(f, v_.snap_f, b, cudaMemcpyDeviceToHost);
@@ -1896,25 +1912,16 @@ std::string Engine::get_snapshot(double *x, double *v, double *f) {
 }
 
 std::string Engine::get_state(double *x, double *v) {
-    // export current x and v (not forces) into the snapshot buffers' copies
-    std::vector<int> orig(N_);
+    // Gathered into original order on the device (the rebuild's scratch holds
+    // both arrays), then one copy each, where seven copies and a scatter on
+    // the host took 0.65 ms at 94,100 atoms.
+    const size_t n3 = 3 * (size_t)N_, bytes = sizeof(double) * n3;
+    launch_state_out(v_, x ? v_.tmp : nullptr, v ? v_.tmp + n3 : nullptr, st_);
+    if (x) touch_pages(x, bytes);
+    if (v) touch_pages(v, bytes);
     cudaStreamSynchronize(st_);
-    cudaMemcpy(orig.data(), v_.orig, sizeof(int) * N_, cudaMemcpyDeviceToHost);
-    std::vector<double> a(N_), b(N_), c(N_);
-    double *src[2][3] = {{v_.x, v_.y, v_.z}, {v_.vx, v_.vy, v_.vz}};
-    double *dst[2] = {x, v};
-    for (int k = 0; k < 2; ++k) {
-        if (!dst[k]) continue;
-        cudaMemcpy(a.data(), src[k][0], sizeof(double) * N_, cudaMemcpyDeviceToHost);
-        cudaMemcpy(b.data(), src[k][1], sizeof(double) * N_, cudaMemcpyDeviceToHost);
-        cudaMemcpy(c.data(), src[k][2], sizeof(double) * N_, cudaMemcpyDeviceToHost);
-        for (int s = 0; s < N_; ++s) {
-            int o = orig[s];
-            dst[k][3 * (size_t)o] = a[s];
-            dst[k][3 * (size_t)o + 1] = b[s];
-            dst[k][3 * (size_t)o + 2] = c[s];
-        }
-    }
+    if (x) cudaMemcpy(x, v_.tmp, bytes, cudaMemcpyDeviceToHost);
+    if (v) cudaMemcpy(v, v_.tmp + n3, bytes, cudaMemcpyDeviceToHost);
     return check("state");
 }
 

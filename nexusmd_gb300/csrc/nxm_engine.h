@@ -249,6 +249,7 @@ private:
 };
 
 void launch_export(const DevView &v, int with_forces, cudaStream_t st);
+void launch_state_out(const DevView &v, double *x, double *vel, cudaStream_t st);
 void launch_decide_rebuild(const DevView &v, int force, cudaStream_t st);
 
 template <typename F>

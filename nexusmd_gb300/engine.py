@@ -248,7 +248,7 @@ class Engine:
         return ms.value
 
     def _get(self, fn):
-        out = np.zeros((self.n_atoms, 3))
+        out = np.empty((self.n_atoms, 3))
         _check(fn(self._h, out), fn.__name__)
         return out
 
@@ -262,8 +262,9 @@ class Engine:
         return self._get(self._L.nxm_get_velocities)
 
     def state(self):
-        x = np.zeros((self.n_atoms, 3))
-        v = np.zeros((self.n_atoms, 3))
+        # one allocation for the two: the allocator keeps it between calls,
+        # where it would hand two of this size back to the system each time
+        x, v = np.empty((2, self.n_atoms, 3))
         _check(self._L.nxm_get_state(self._h, x, v), "get_state")
         return x, v
 
