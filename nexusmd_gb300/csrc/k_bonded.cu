@@ -231,11 +231,11 @@ __global__ void __launch_bounds__(256) k_bonded(DevView v, int energy, int pairs
 int launch_bonded(const DevView &v, int energy, cudaStream_t st, int pairs) {
     int n = v.nb + v.na + v.nt + (pairs ? v.nex + v.nxc : 0);  // disabled kinds arrive with a zero count
     if (n == 0) return 0;
-    int nb = (n + 255) / 256;
+    const int t = thread_block(n), nb = (n + t - 1) / t;
     if (v.mixed)
-        k_bonded<float, long long><<<nb, 256, 0, st>>>(v, energy, pairs);
+        k_bonded<float, long long><<<nb, t, 0, st>>>(v, energy, pairs);
     else
-        k_bonded<double, double><<<nb, 256, 0, st>>>(v, energy, pairs);
+        k_bonded<double, double><<<nb, t, 0, st>>>(v, energy, pairs);
     return 1;
 }
 

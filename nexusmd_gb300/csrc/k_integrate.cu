@@ -199,23 +199,24 @@ __global__ void k_state_out(DevView v, double *x, double *vel) {
 }
 
 void launch_state_out(const DevView &v, double *x, double *vel, cudaStream_t st) {
-    if (v.N) k_state_out<<<(v.N + 255) / 256, 256, 0, st>>>(v, x, vel);
+    const int t = thread_block(v.N);
+    if (v.N) k_state_out<<<(v.N + t - 1) / t, t, 0, st>>>(v, x, vel);
 }
 
 void launch_integrate(const DevView &v, double dt, int report, cudaStream_t st) {
-    int nb = (v.N + 255) / 256;
+    const int t = thread_block(v.N), nb = (v.N + t - 1) / t;
     if (v.mixed)
-        k_integrate<long long><<<nb, 256, 0, st>>>(v, dt, report);
+        k_integrate<long long><<<nb, t, 0, st>>>(v, dt, report);
     else
-        k_integrate<double><<<nb, 256, 0, st>>>(v, dt, report);
+        k_integrate<double><<<nb, t, 0, st>>>(v, dt, report);
 }
 
 void launch_export(const DevView &v, int with_forces, cudaStream_t st) {
-    int nb = (v.N + 255) / 256;
+    const int t = thread_block(v.N), nb = (v.N + t - 1) / t;
     if (v.mixed)
-        k_export<long long><<<nb, 256, 0, st>>>(v, with_forces);
+        k_export<long long><<<nb, t, 0, st>>>(v, with_forces);
     else
-        k_export<double><<<nb, 256, 0, st>>>(v, with_forces);
+        k_export<double><<<nb, t, 0, st>>>(v, with_forces);
 }
 
 void launch_snapshot_forces(const DevView &v, cudaStream_t st) { launch_export(v, 1, st); }

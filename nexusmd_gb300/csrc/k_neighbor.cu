@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_cellsort(DevView v) {
     __shared__ float s_pos[kSortWarps][3][kSortMax];
     const unsigned full = 0xffffffffu;
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int c = blockIdx.x * kSortWarps + warp;
+    int c = blockIdx.x * (blockDim.x >> 5) + warp;
     if (c >= v.total_cells) return;
     int a = v.cell_start[c], n = v.cell_start[c + 1] - a;
     // the cell's count and fill words, done with, start the next rebuild at zero
@@ -331,26 +331,31 @@ __global__ void k_remap(DevView v) {
 static inline int blocks(long long n, int t) { return (int)((n + t - 1) / t); }
 
 void launch_derive_inputs(const DevView &v, cudaStream_t st) {
-    k_derive<<<blocks(v.N, 256), 256, 0, st>>>(v);
+    const int t = thread_block(v.N);
+    k_derive<<<blocks(v.N, t), t, 0, st>>>(v);
 }
 
 void launch_remap_terms(const DevView &v, cudaStream_t st) {
     long long n = (long long)v.nb + v.na + v.nt + v.nex + v.nxc;
-    if (n > 0) k_remap<<<blocks(n, 256), 256, 0, st>>>(v);
+    const int t = thread_block(n);
+    if (n > 0) k_remap<<<blocks(n, t), t, 0, st>>>(v);
 }
 
 void launch_nlist_order(const DevView &v, cudaStream_t st) {
-    k_assign<<<blocks(v.N, 256), 256, 0, st>>>(v);
+    const int t = thread_block(v.N);
+    const int w = v.total_cells >= 2 * 152 * kSortWarps ? kSortWarps : 1;
+    k_assign<<<blocks(v.N, t), t, 0, st>>>(v);
     k_scan<<<1, 1024, 0, st>>>(v.flags, v.cell_count, v.cell_start, v.total_cells);
-    k_scatter<<<blocks(v.N, 256), 256, 0, st>>>(v);
-    k_cellsort<<<blocks(v.total_cells, kSortWarps), kSortWarps * 32, 0, st>>>(v);
-    k_permute_gather<<<blocks(v.N, 256), 256, 0, st>>>(v);
-    k_permute_scatter<<<blocks(v.N, 256), 256, 0, st>>>(v);
+    k_scatter<<<blocks(v.N, t), t, 0, st>>>(v);
+    k_cellsort<<<blocks(v.total_cells, w), w * 32, 0, st>>>(v);
+    k_permute_gather<<<blocks(v.N, t), t, 0, st>>>(v);
+    k_permute_scatter<<<blocks(v.N, t), t, 0, st>>>(v);
 }
 
 void launch_nlist_lists(const DevView &v, cudaStream_t st) {
     long long nt = (long long)v.nb + v.na + v.nt + v.nex + v.nxc;
-    if (nt > 0) k_remap<<<blocks(nt, 256), 256, 0, st>>>(v);
+    const int t = thread_block(nt);
+    if (nt > 0) k_remap<<<blocks(nt, t), t, 0, st>>>(v);
     launch_build(v, st);
 }
 

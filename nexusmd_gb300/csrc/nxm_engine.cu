@@ -1497,7 +1497,8 @@ std::string Engine::stage_state(const double *xyz, double *dx, double *dy, doubl
     cudaMemcpyAsync(stage3_, xyz, sizeof(double) * 3 * (size_t)N_, cudaMemcpyHostToDevice, st_copy_);
     cudaEventRecord(ev_staged_, st_copy_);
     cudaStreamWaitEvent(st_, ev_staged_, 0);
-    if (N_ > 0) k_state_to_slots<<<(N_ + 255) / 256, 256, 0, st_>>>(v_, stage3_, dx, dy, dz);
+    const int t = thread_block(N_);
+    if (N_ > 0) k_state_to_slots<<<(N_ + t - 1) / t, t, 0, st_>>>(v_, stage3_, dx, dy, dz);
     cudaEventRecord(ev_stage_free_, st_);
     stage_used_ = true;
     return check("state upload");
