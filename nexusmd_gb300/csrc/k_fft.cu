@@ -27,6 +27,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "nxm_chain.cuh"
 #include "nxm_fft.h"
 #include "nxm_view.h"
 
@@ -380,6 +381,7 @@ __global__ void __launch_bounds__(1024) k_fft_plane_fwd(const __grid_constant__ 
                                                         int twcap, int qcap, int scr) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *twy = reinterpret_cast<C *>(smem_raw);
+    chain_link();
     const FftWork w = ONE ? FftWork{0, (int)blockIdx.x} : work[blockIdx.x];
     const FftSysDev &F = ONE ? one : fs[w.sys];
     const int K1 = F.K[1], K2 = F.K[2], Kh = F.Kh, x = w.unit;
@@ -421,6 +423,7 @@ __global__ void __launch_bounds__(1024) k_fft_plane_inv(const __grid_constant__ 
     using T = typename Cx<C>::R;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *twy = reinterpret_cast<C *>(smem_raw);
+    chain_link();
     const FftWork w = ONE ? FftWork{0, (int)blockIdx.x} : work[blockIdx.x];
     const FftSysDev &F = ONE ? one : fs[w.sys];
     const int K1 = F.K[1], K2 = F.K[2], Kh = F.Kh, x = w.unit;
@@ -624,6 +627,7 @@ __global__ void __launch_bounds__(256) k_fft_z_fwd(const __grid_constant__ DevVi
     using T = typename Cx<C>::R;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *tw = reinterpret_cast<C *>(smem_raw);
+    chain_link();
     const FftWork w = ONE ? FftWork{0, (int)blockIdx.x} : work[blockIdx.x];
     const FftSysDev &F = ONE ? one : fs[w.sys];
     const int n = F.K[2], Kh = F.Kh, ld = n | 1;
@@ -664,6 +668,7 @@ __global__ void __launch_bounds__(256) k_fft_y(const __grid_constant__ DevView v
                                                int kmax) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *tw = reinterpret_cast<C *>(smem_raw);
+    chain_link();
     const FftWork w = ONE ? FftWork{0, (int)blockIdx.x} : work[blockIdx.x];
     const FftSysDev &F = ONE ? one : fs[w.sys];
     const int n = F.K[1], Kh = F.Kh, ld = n | 1;
@@ -696,6 +701,7 @@ __global__ void __launch_bounds__(256) k_fft_x_conv(const __grid_constant__ DevV
     using T = typename Cx<C>::R;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *tw = reinterpret_cast<C *>(smem_raw);
+    chain_link();
     const FftWork w = ONE ? FftWork{0, (int)blockIdx.x} : work[blockIdx.x];
     const FftSysDev &F = ONE ? one : fs[w.sys];
     const int n = F.K[0], K1 = F.K[1], Kh = F.Kh, ld = n | 1;
@@ -787,6 +793,7 @@ __global__ void __launch_bounds__(256) k_fft_z_inv(const __grid_constant__ DevVi
     using T = typename Cx<C>::R;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *tw = reinterpret_cast<C *>(smem_raw);
+    chain_link();
     const FftWork w = ONE ? FftWork{0, (int)blockIdx.x} : work[blockIdx.x];
     const FftSysDev &F = ONE ? one : fs[w.sys];
     const int n = F.K[2], Kh = F.Kh, ld = n | 1;
@@ -823,19 +830,22 @@ __global__ void __launch_bounds__(256) k_fft_z_inv(const __grid_constant__ DevVi
 template <typename C, typename Acc, typename ET, bool ONE>
 static void run(const DevView &v, const FftPlan &p, int energy, cudaStream_t st) {
     const FftSysDev &F = ONE ? p.hsys[0] : FftSysDev{};
+    const bool c = p.chained;
     if (p.plane) {
-        k_fft_plane_fwd<C, Acc, ONE>
-            <<<p.npl, p.plane_threads, p.smem_plane, st>>>(v, p.dsys, F, p.pwork, p.twcap, p.qcap, p.scr);
-        k_fft_x_conv<C, ET, ONE><<<p.nx, p.cthreads, p.smem_x, st>>>(v, p.dsys, F, p.xwork, p.cols, p.kmax, energy);
-        k_fft_plane_inv<C, ONE>
-            <<<p.npl, p.plane_threads, p.smem_plane, st>>>(v, p.dsys, F, p.pwork, p.twcap, p.qcap, p.scr);
+        launch_link(c, k_fft_plane_fwd<C, Acc, ONE>, p.npl, p.plane_threads, p.smem_plane, st, v, p.dsys, F, p.pwork,
+                    p.twcap, p.qcap, p.scr);
+        launch_link(c, k_fft_x_conv<C, ET, ONE>, p.nx, p.cthreads, p.smem_x, st, v, p.dsys, F, p.xwork, p.cols, p.kmax,
+                    energy);
+        launch_link(c, k_fft_plane_inv<C, ONE>, p.npl, p.plane_threads, p.smem_plane, st, v, p.dsys, F, p.pwork,
+                    p.twcap, p.qcap, p.scr);
         return;
     }
-    k_fft_z_fwd<C, Acc, ONE><<<p.nz, p.zthreads, p.smem_z, st>>>(v, p.dsys, F, p.zwork, p.zlines, p.kmax);
-    k_fft_y<C, false, ONE><<<p.ny, p.cthreads, p.smem_y, st>>>(v, p.dsys, F, p.ywork, p.cols, p.kmax);
-    k_fft_x_conv<C, ET, ONE><<<p.nx, p.cthreads, p.smem_x, st>>>(v, p.dsys, F, p.xwork, p.cols, p.kmax, energy);
-    k_fft_y<C, true, ONE><<<p.ny, p.cthreads, p.smem_y, st>>>(v, p.dsys, F, p.ywork, p.cols, p.kmax);
-    k_fft_z_inv<C, ONE><<<p.nz, p.zthreads, p.smem_z, st>>>(v, p.dsys, F, p.zwork, p.zlines, p.kmax);
+    launch_link(c, k_fft_z_fwd<C, Acc, ONE>, p.nz, p.zthreads, p.smem_z, st, v, p.dsys, F, p.zwork, p.zlines, p.kmax);
+    launch_link(c, k_fft_y<C, false, ONE>, p.ny, p.cthreads, p.smem_y, st, v, p.dsys, F, p.ywork, p.cols, p.kmax);
+    launch_link(c, k_fft_x_conv<C, ET, ONE>, p.nx, p.cthreads, p.smem_x, st, v, p.dsys, F, p.xwork, p.cols, p.kmax,
+                energy);
+    launch_link(c, k_fft_y<C, true, ONE>, p.ny, p.cthreads, p.smem_y, st, v, p.dsys, F, p.ywork, p.cols, p.kmax);
+    launch_link(c, k_fft_z_inv<C, ONE>, p.nz, p.zthreads, p.smem_z, st, v, p.dsys, F, p.zwork, p.zlines, p.kmax);
 }
 
 template <typename C, typename Acc, typename ET>

@@ -33,6 +33,7 @@
 #include <string>
 
 #include "../../include/nxm.h"
+#include "nxm_chain.cuh"
 #include "nxm_fft.h"
 #include "nxm_spread.cuh"
 #include "nxm_view.h"
@@ -111,6 +112,7 @@ __device__ __forceinline__ double modulus2(int k, int K) {
 constexpr int kAxisBlocks = 3 * kStaticMaxK / 32;
 
 __global__ void __launch_bounds__(256) k_noalloc_setup(unsigned char *scr, Geometry g) {
+    chain_link();
     if (blockIdx.x >= kAxisBlocks) {
         int4 *acc = region<int4>(scr, kOffAcc);
         const int n = (g.K[0] * g.K[1] * g.K[2] + 3) / 4;  // (the region holds whole int4)
@@ -155,6 +157,7 @@ constexpr int kAtoms = 8, kSpreadBlockWarps = 4;
 __global__ void __launch_bounds__(kSpreadBlockWarps * 32) k_noalloc_spread(unsigned char *scr, Geometry g,
                                                                            const double *xyz, const double *charge,
                                                                            int n, int nspread) {
+    chain_link();
     if ((int)blockIdx.x >= nspread) {
         const double2 *ax = region<double2>(scr, kOffAxis), *ay = ax + kStaticMaxK, *az = ay + kStaticMaxK;
         float *et = region<float>(scr, kOffEterm);
@@ -199,6 +202,7 @@ constexpr int kGatherThreads = 64;
 __global__ void __launch_bounds__(kGatherThreads) k_noalloc_gather(unsigned char *scr, Geometry g, const double *xyz,
                                                                    const double *charge, int n, double *force,
                                                                    double *energy) {
+    chain_link();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) *energy = (double)region<long long>(scr, kOffE)[E_RECIP] * kEnergyUnscale;
     if (i >= n) return;
@@ -354,10 +358,14 @@ extern "C" int nxm_pme_reciprocal_noalloc(const double *xyz, const double *charg
     k_noalloc_setup<<<kAxisBlocks + 152, 256, 0, st>>>(scr, g);
     const int nspread = (n_atoms + kSpreadBlockWarps * kAtoms - 1) / (kSpreadBlockWarps * kAtoms);
     const int neterm = (int)std::min<long long>((v.total_cgrid + kSpreadBlockWarps * 32 - 1) / (kSpreadBlockWarps * 32), 608);
-    k_noalloc_spread<<<nspread + neterm, kSpreadBlockWarps * 32, 0, st>>>(scr, g, xyz, charge, n_atoms, nspread);
+    // (the first kernel is an ordinary launch: it follows whatever the caller
+    // put on the stream)
+    plan.chained = true;
+    launch_link(true, k_noalloc_spread, nspread + neterm, kSpreadBlockWarps * 32, 0, st, scr, g, xyz, charge, n_atoms,
+                nspread);
     launch_fft_convolve(v, plan, 1, st);
-    k_noalloc_gather<<<std::max(1, (n_atoms + kGatherThreads - 1) / kGatherThreads), kGatherThreads, 0, st>>>(
-        scr, g, xyz, charge, n_atoms, force, energy);
+    launch_link(true, k_noalloc_gather, std::max(1, (n_atoms + kGatherThreads - 1) / kGatherThreads), kGatherThreads, 0,
+                st, scr, g, xyz, charge, n_atoms, force, energy);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(NXM_ERR_CUDA, std::string(fn) + "launch failed: " + cudaGetErrorString(e));
     return NXM_OK;

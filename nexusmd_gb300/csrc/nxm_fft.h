@@ -55,6 +55,7 @@ struct FftPlan {
     int nz = 0, ny = 0, nx = 0;
     int zlines = 16;    // real lines per block in the z passes (even)
     int cols = 8;       // columns per block in the y and x passes (a power of two)
+    bool chained = false;  // the kernels are links of a chain (nxm_chain.cuh)
     int zthreads = 256, cthreads = 256;  // threads per block of the z, and of the y and x passes
     size_t smem_z = 0, smem_y = 0, smem_x = 0;
     int kmax = 0;
