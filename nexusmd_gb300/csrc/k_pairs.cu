@@ -586,12 +586,13 @@ __device__ __forceinline__ void near_cutoff(const DevView &v, const SysDev &S, c
 // pipe for two).  An entry costs one load of j, one decoding and one set of
 // packed operations for two interactions, 12% of which the other atom's
 // share of the list adds: 145 -> 132 us at 94,100 atoms against a list per
-// atom, 189 -> 141 us with the switching function at 74,400, 101 -> 88 M warp
+// atom, 189 -> 129 us with the switching function at 74,400, 101 -> 88 M warp
 // instructions.  Of its walk 57% of the cycles issue; the rest is the staging
 // before it and a block's last pairs.
-// SW: some system of the batch uses the switching function.
+// SW: some system of the batch uses the switching function; W: warps per block
+// (pairs_warps).
 template <bool ENERGY, bool SW, int W>
-__global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_pairs_mixed(const __grid_constant__ DevView v) {
+__global__ void __launch_bounds__(W * 32, W <= kHoodWarps ? 2 : 1) k_pairs_mixed(const __grid_constant__ DevView v) {
     extern __shared__ __align__(16) unsigned char smem[];
     const unsigned full = 0xffffffffu;
     CellGroup G = v.groups[blockIdx.x];
@@ -1120,7 +1121,6 @@ constexpr size_t kTileStatic = 25 * kRowCells * sizeof(float4) + 16;
 // neighbourhoods -- one-cell groups of large cells -- need the latter.)
 static bool wide(size_t dynamic_smem) { return 2 * (dynamic_smem + kTileStatic + 1024) > 228 * 1024; }
 static int build_warps(int cap) { return wide(smem_build(cap, kHoodWarps)) ? 2 * kHoodWarps : kHoodWarps; }
-static int pair_warps(int cap) { return wide(smem_pairs(cap)) ? 2 * kHoodWarps : kHoodWarps; }
 
 template <int W>
 static void set_build_smem(int b) {
@@ -1128,12 +1128,24 @@ static void set_build_smem(int b) {
     cudaFuncSetAttribute(k_build<false, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
 }
 
-template <int W>
+// Warps per block of the mixed pair kernel, two blocks per SM (or one of twice
+// as many, `wide`): 16 at 64 registers per thread; 14 at 72 or 12 at 80 where
+// what the kernel carries (the switch, the energies) would spill.  Measured
+// with 16, 14 and 12: the switch at 74,400 atoms 142, 132, 129 us, steps with
+// energies 262, 247, 242; without it at 94,100 atoms 133, 134, 133 us, steps
+// with energies 0.268, 0.266, 0.269 ms; one block per SM, 32 systems 579, 570,
+// 574 us, 473,400 atoms 914, 911, 930.
+constexpr int pairs_warps(bool energy, bool sw, bool wide) {
+    return sw ? (wide ? 24 : 12) : wide ? 28 : energy ? 14 : 16;
+}
+
+template <bool WIDE>
 static void set_pairs_smem(int m) {
-    cudaFuncSetAttribute(k_pairs_mixed<true, false, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
-    cudaFuncSetAttribute(k_pairs_mixed<false, false, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
-    cudaFuncSetAttribute(k_pairs_mixed<true, true, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
-    cudaFuncSetAttribute(k_pairs_mixed<false, true, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
+    auto set = [&](auto kernel) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, m); };
+    set(k_pairs_mixed<true, false, pairs_warps(true, false, WIDE)>);
+    set(k_pairs_mixed<false, false, pairs_warps(false, false, WIDE)>);
+    set(k_pairs_mixed<true, true, pairs_warps(true, true, WIDE)>);
+    set(k_pairs_mixed<false, true, pairs_warps(false, true, WIDE)>);
 }
 
 // The dynamic shared-memory limit is a per-kernel attribute shared by every
@@ -1146,9 +1158,9 @@ void tiles_set_smem(int cap) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= kMaxSmemDevices) dev = 0;
-    const int bw = build_warps(cap), pw = pair_warps(cap);
+    const int bw = build_warps(cap);
     const int b = (int)smem_build(cap, bw), m = (int)smem_pairs(cap), d = (int)smem_pairs64(cap);
-    const int bi = bw == kHoodWarps ? 0 : 1, pi = pw == kHoodWarps ? 0 : 1;
+    const int bi = bw == kHoodWarps ? 0 : 1, pi = wide(smem_pairs(cap)) ? 1 : 0;
     std::lock_guard<std::mutex> lock(mu);
     // launches up to 48 KB, static shared memory included, need no attribute
     constexpr int kFree = 48 * 1024 - (int)kTileStatic - 1024;
@@ -1161,9 +1173,9 @@ void tiles_set_smem(int cap) {
     }
     if (m > kFree && m > seen_pairs[pi][dev]) {
         if (pi)
-            set_pairs_smem<2 * kHoodWarps>(m);
+            set_pairs_smem<true>(m);
         else
-            set_pairs_smem<kHoodWarps>(m);
+            set_pairs_smem<false>(m);
         seen_pairs[pi][dev] = m;
     }
     if (d > kFree && d > seen_pairs64[dev]) {
@@ -1192,30 +1204,27 @@ void launch_build(const DevView &v, cudaStream_t st) {
         launch_build_w<2 * kHoodWarps>(v, st);
 }
 
-template <int W>
+template <bool ENERGY, bool SW, bool WIDE>
+static void launch_pairs_variant(const DevView &v, cudaStream_t st) {
+    constexpr int W = pairs_warps(ENERGY, SW, WIDE);
+    k_pairs_mixed<ENERGY, SW, W><<<v.ngroups, W * 32, smem_pairs(v.hood_cap), st>>>(v);
+}
+
+template <bool WIDE>
 static void launch_pairs_mixed(const DevView &v, int energy, cudaStream_t st) {
-    const int g = v.ngroups, t = W * 32;
-    const size_t sm = smem_pairs(v.hood_cap);
-    if (v.any_switch) {
-        if (energy)
-            k_pairs_mixed<true, true, W><<<g, t, sm, st>>>(v);
-        else
-            k_pairs_mixed<false, true, W><<<g, t, sm, st>>>(v);
-    } else {
-        if (energy)
-            k_pairs_mixed<true, false, W><<<g, t, sm, st>>>(v);
-        else
-            k_pairs_mixed<false, false, W><<<g, t, sm, st>>>(v);
-    }
+    if (v.any_switch)
+        energy ? launch_pairs_variant<true, true, WIDE>(v, st) : launch_pairs_variant<false, true, WIDE>(v, st);
+    else
+        energy ? launch_pairs_variant<true, false, WIDE>(v, st) : launch_pairs_variant<false, false, WIDE>(v, st);
 }
 
 void launch_pairs(const DevView &v, int energy, cudaStream_t st) {
     if (v.N == 0 || v.ngroups == 0) return;
     if (v.mixed) {
-        if (pair_warps(v.hood_cap) == kHoodWarps)
-            launch_pairs_mixed<kHoodWarps>(v, energy, st);
+        if (wide(smem_pairs(v.hood_cap)))
+            launch_pairs_mixed<true>(v, energy, st);
         else
-            launch_pairs_mixed<2 * kHoodWarps>(v, energy, st);
+            launch_pairs_mixed<false>(v, energy, st);
         return;
     }
     // A group's atoms may be dealt to several blocks, each staging the
