@@ -350,18 +350,14 @@ void launch_nlist_order(const DevView &v, cudaStream_t st) {
     k_cellsort<<<blocks(v.total_cells, w), w * 32, 0, st>>>(v);
     k_permute_gather<<<blocks(v.N, t), t, 0, st>>>(v);
     k_permute_scatter<<<blocks(v.N, t), t, 0, st>>>(v);
-}
-
-void launch_nlist_lists(const DevView &v, cudaStream_t st) {
     long long nt = (long long)v.nb + v.na + v.nt + v.nex + v.nxc;
-    const int t = thread_block(nt);
-    if (nt > 0) k_remap<<<blocks(nt, t), t, 0, st>>>(v);
-    launch_build(v, st);
+    const int tt = thread_block(nt);
+    if (nt > 0) k_remap<<<blocks(nt, tt), tt, 0, st>>>(v);
 }
 
 void launch_nlist_rebuild(const DevView &v, cudaStream_t st) {
     launch_nlist_order(v, st);
-    launch_nlist_lists(v, st);
+    launch_build(v, st);
 }
 
 }  // namespace nxm

@@ -42,15 +42,16 @@ __global__ void k_decide(DevView v, int force) {
 void launch_decide_rebuild(const DevView &v, int force, cudaStream_t st) { k_decide<<<1, 1, 0, st>>>(v, force); }
 
 // The same decision inside a step graph: it also opens or closes the
-// graph's conditional rebuild node.
-__global__ void k_decide_graph(DevView v, cudaGraphConditionalHandle h) {
+// graph's conditional nodes (slot order; lists, where they have their own).
+__global__ void k_decide_graph(DevView v, cudaGraphConditionalHandle order, cudaGraphConditionalHandle lists) {
     Flags *f = v.flags;
     int rb = f->since >= f->interval || f->skin_hit;
     f->rebuild = rb;
     f->skin_hit = 0;
     f->since = rb ? 1 : f->since + 1;
     if (rb) f->nrebuild += 1;
-    cudaGraphSetConditional(h, rb ? 1u : 0u);
+    cudaGraphSetConditional(order, rb ? 1u : 0u);
+    if (lists != order) cudaGraphSetConditional(lists, rb ? 1u : 0u);
 }
 
 // Context creation: positions given per atom as (x, y, z) into x, y, z;
@@ -1570,6 +1571,8 @@ std::string Engine::build_graph(double dt, int report) {
     return r;
 }
 
+constexpr int kSplitAtoms = 10000;
+
 std::string Engine::build_graph_timed(double dt, int report) {
     StepGraph &G = graph_[report];
     const DevView vv = view_for(report);
@@ -1579,64 +1582,94 @@ std::string Engine::build_graph_timed(double dt, int report) {
     const cudaStreamCaptureMode mode = cudaStreamCaptureModeThreadLocal;
     cudaGraph_t g = nullptr, captured = nullptr;
     auto fail_capture = [&](const char *what, cudaError_t e) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st_, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
-            cudaStreamEndCapture(st_, &captured);
+        for (cudaStream_t st : {st_, st_pme_}) {
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
+                cudaStreamEndCapture(st, &captured);
+        }
         cudaGetLastError();
         return std::string("step graph: ") + what + ": " + cudaGetErrorString(e);
     };
     cudaError_t e = cudaGraphCreate(&g, 0);
     if (e != cudaSuccess) return fail_capture("create", e);
     G.graph = g;
-    cudaGraphConditionalHandle h;
-    e = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault);
+    const bool split = N_ >= kSplitAtoms;  // the lists in a conditional node of their own (below)
+    cudaGraphConditionalHandle h_order, h_lists;
+    e = cudaGraphConditionalHandleCreate(&h_order, g, 0, cudaGraphCondAssignDefault);
+    h_lists = h_order;
+    if (e == cudaSuccess && split) e = cudaGraphConditionalHandleCreate(&h_lists, g, 0, cudaGraphCondAssignDefault);
     if (e != cudaSuccess) return fail_capture("conditional handle", e);
-    // head: energy reset and the decision
-    e = cudaStreamBeginCaptureToGraph(st_, g, nullptr, nullptr, 0, mode);
+    // Captures what `launch` puts on stream st behind the nodes `after`;
+    // returns the nodes it ends in.
+    using Nodes = std::vector<cudaGraphNode_t>;
+    auto captured_after = [&](cudaStream_t st, const Nodes &after, auto &&launch, Nodes &end) {
+        cudaError_t r = cudaStreamBeginCaptureToGraph(st, g, after.data(), nullptr, after.size(), mode);
+        if (r != cudaSuccess) return r;
+        launch();
+        cudaStreamCaptureStatus cs;
+        const cudaGraphNode_t *deps = nullptr;
+        size_t nd = 0;
+        r = cudaStreamGetCaptureInfo(st, &cs, nullptr, nullptr, &deps, nullptr, &nd);
+        if (r == cudaSuccess) end.assign(deps, deps + nd);
+        const cudaError_t q = cudaStreamEndCapture(st, &captured);
+        return r != cudaSuccess ? r : q;
+    };
+    // A conditional node behind `after` whose body is what `launch` enqueues.
+    auto conditional = [&](cudaGraphConditionalHandle h, const Nodes &after, auto &&launch, Nodes &end) {
+        cudaGraphNodeParams cp = {};
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = h;
+        cp.conditional.type = cudaGraphCondTypeIf;
+        cp.conditional.size = 1;
+        cudaGraphNode_t node;
+        cudaError_t r = cudaGraphAddNode(&node, g, after.data(), nullptr, after.size(), &cp);
+        if (r != cudaSuccess) return r;
+        r = cudaStreamBeginCaptureToGraph(st_, cp.conditional.phGraph_out[0], nullptr, nullptr, 0, mode);
+        if (r != cudaSuccess) return r;
+        launch();
+        r = cudaStreamEndCapture(st_, &captured);
+        end.assign(1, node);
+        return r;
+    };
+    // Energy reset and the decision, the charge grid cleared beside them; the
+    // new slot order, when the decision asks for one; behind it the PME chain
+    // on a branch of its own, and on the other the lists (when asked for), the
+    // bonded terms and the pairs; the update behind both.  The PME chain needs
+    // no lists, so on a step that rebuilds it runs beside their build: 20 steps
+    // at 94,100 atoms 5.46 -> 5.33 ms, 50 at 23,800 5.13 -> 5.04.  A conditional
+    // node costs four microseconds whether or not it runs, more than the build
+    // of a small system lends: 2,700 atoms 44 us a step with one, 49 with two.
+    Nodes head, grid, order, lists, pme, forces, last;
+    const bool with_pme = (vv.force_mask & NXM_FORCE_NONBONDED) && plan_.nz;
+    e = captured_after(st_, {}, [&] {
+        if (report) cudaMemsetAsync(vv.E, 0, sizeof(long long) * v_.S * E_SLOTS, st_);
+        k_decide_graph<<<1, 1, 0, st_>>>(vv, h_order, h_lists);
+    }, head);
     if (e != cudaSuccess) return fail_capture("capture head", e);
-    // (the charge grid is cleared beside the decision)
-    cudaEventRecord(ev_fork_, st_);
-    cudaStreamWaitEvent(st_pme_, ev_fork_, 0);
-    launch_clear_grid(vv, st_pme_);
-    cudaEventRecord(ev_join_, st_pme_);
-    if (report) cudaMemsetAsync(vv.E, 0, sizeof(long long) * v_.S * E_SLOTS, st_);
-    k_decide_graph<<<1, 1, 0, st_>>>(vv, h);
-    cudaStreamWaitEvent(st_, ev_join_, 0);
-    cudaStreamCaptureStatus cs;
-    const cudaGraphNode_t *deps = nullptr;
-    size_t nd = 0;
-    e = cudaStreamGetCaptureInfo(st_, &cs, nullptr, nullptr, &deps, nullptr, &nd);
-    if (e != cudaSuccess) return fail_capture("capture info", e);
-    std::vector<cudaGraphNode_t> head(deps, deps + nd);
-    e = cudaStreamEndCapture(st_, &captured);
-    if (e != cudaSuccess) return fail_capture("end head", e);
-    // the conditional rebuild node and its body
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeIf;
-    cp.conditional.size = 1;
-    cudaGraphNode_t cnode;
-    e = cudaGraphAddNode(&cnode, g, head.data(), nullptr, head.size(), &cp);
-    if (e != cudaSuccess) return fail_capture("conditional node", e);
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    e = cudaStreamBeginCaptureToGraph(st_, body, nullptr, nullptr, 0, mode);
-    if (e != cudaSuccess) return fail_capture("capture rebuild", e);
-    launch_nlist_rebuild(vv, st_);
-    e = cudaStreamEndCapture(st_, &captured);
-    if (e != cudaSuccess) return fail_capture("end rebuild", e);
-    // tail: forces and update, after the conditional node
-    e = cudaStreamBeginCaptureToGraph(st_, g, &cnode, nullptr, 1, mode);
-    if (e != cudaSuccess) return fail_capture("capture tail", e);
-    // PME as a parallel branch on the second stream, joined before the update
-    cudaEventRecord(ev_fork_, st_);
-    cudaStreamWaitEvent(st_pme_, ev_fork_, 0);
-    force_launches(vv, plan_, report ? 1 : 0, st_, st_pme_, true);
-    cudaEventRecord(ev_join_, st_pme_);
-    cudaStreamWaitEvent(st_, ev_join_, 0);
-    launch_integrate(vv, dt, report >= 2 ? 2 : report, st_);
-    e = cudaStreamEndCapture(st_, &captured);
-    if (e != cudaSuccess) return fail_capture("end tail", e);
+    if (with_pme) {
+        e = captured_after(st_pme_, {}, [&] { launch_clear_grid(vv, st_pme_); }, grid);
+        if (e != cudaSuccess) return fail_capture("capture grid", e);
+    }
+    e = conditional(h_order, head, [&] {
+        launch_nlist_order(vv, st_);
+        if (!split) launch_build(vv, st_);
+    }, order);
+    if (e != cudaSuccess) return fail_capture("slot order node", e);
+    if (with_pme) {
+        grid.insert(grid.end(), order.begin(), order.end());
+        e = captured_after(st_pme_, grid, [&] { launch_pme(vv, plan_, report ? 1 : 0, st_pme_, true); }, pme);
+        if (e != cudaSuccess) return fail_capture("capture PME", e);
+    }
+    lists = order;
+    if (split) {
+        e = conditional(h_lists, order, [&] { launch_build(vv, st_); }, lists);
+        if (e != cudaSuccess) return fail_capture("lists node", e);
+    }
+    e = captured_after(st_, lists, [&] { force_launches(vv, plan_, report ? 1 : 0, st_, st_pme_, true, true); }, forces);
+    if (e != cudaSuccess) return fail_capture("capture forces", e);
+    forces.insert(forces.end(), pme.begin(), pme.end());
+    e = captured_after(st_, forces, [&] { launch_integrate(vv, dt, report >= 2 ? 2 : report, st_); }, last);
+    if (e != cudaSuccess) return fail_capture("capture update", e);
     e = cudaGraphInstantiate(&G.exec, g, 0);
     if (e != cudaSuccess) return fail_capture("instantiate", e);
     G.dt = dt;
@@ -1658,7 +1691,7 @@ int Engine::forced_evaluation(const DevView &vv, int energy) {
         launch_pme(vv, plan_, energy, st_pme_);
         cudaEventRecord(ev_join_, st_pme_);
     }
-    launch_nlist_lists(vv, st_);
+    launch_build(vv, st_);
     const int n = force_launches(vv, plan_, energy, st_, pme ? st_pme_ : nullptr, false, pme);
     if (pme) cudaStreamWaitEvent(st_, ev_join_, 0);
     return n;

@@ -151,9 +151,9 @@ public:
 
 private:
     // One step as a CUDA graph: energy reset (report steps), the list
-    // decision, a conditional node whose body is the rebuild sequence (run
-    // only when the decision kernel sets it), the force kernels and the
-    // update.  One graph per report flag, rebuilt when dt changes.
+    // decision, two conditional nodes for the parts of a rebuild (run only
+    // when the decision kernel sets them), the force kernels on two branches
+    // and the update.  One graph per report kind, rebuilt when dt changes.
     struct StepGraph {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;

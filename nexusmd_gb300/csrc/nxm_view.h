@@ -128,10 +128,9 @@ void launch_exclusions_count(const ExclBuild &b, cudaStream_t st);
 void launch_exclusions_fill(const ExclBuild &b, int *elst, int2 *pairs, cudaStream_t st);
 
 // kernel launchers (one per .cu file group)
-// the rebuild in two parts: the slot order with the per-atom state in it, and
-// what is indexed by it (term indices, lists); launch_nlist_rebuild: both
+// the rebuild in two parts: the slot order with the per-atom state and the
+// terms' indices in it, and the lists (launch_build); launch_nlist_rebuild: both
 void launch_nlist_order(const DevView &v, cudaStream_t st);
-void launch_nlist_lists(const DevView &v, cudaStream_t st);
 void launch_nlist_rebuild(const DevView &v, cudaStream_t st);
 void launch_build(const DevView &v, cudaStream_t st);
 void tiles_set_smem(int hood_cap);
