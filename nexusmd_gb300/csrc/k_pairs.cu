@@ -783,8 +783,8 @@ __global__ void __launch_bounds__(W * 32, W <= kHoodWarps ? 2 : 1) k_pairs_mixed
 //    terms as erf (an entire function of r^2 over r, Taylor rows in a table
 //    that stays in L1) subtracted from the bare Coulomb term: about 40 FP64
 //    instructions per pair, where erfc, exp, sqrt and the divisions took
-//    about 240 per list entry.  23,800 atoms: 5,390 -> 567 us, the FP64 pipe
-//    busy 83% of the kernel's active cycles; 2,700 atoms: 727 -> 96 us.
+//    about 240 per list entry.  23,800 atoms: 5,390 -> 554 us, the FP64 pipe
+//    busy 79% of the kernel's active cycles; 2,700 atoms: 727 -> 92 us.
 // The pair set is decided on the exact r^2 of the reference's list.
 
 constexpr int kWarps64 = 8;
@@ -797,12 +797,15 @@ __device__ __forceinline__ double negated(double x) {
 }
 
 // min_image() with |d| > L/2 compared as integers (the order of non-negative
-// doubles), and no FP64 addition issued for a warp none of whose lanes shifts.
+// doubles), and no FP64 addition issued for a warp none of whose lanes shifts
+// (volatile: else both sums are formed ahead of the vote and one is selected,
+// a fifth of the kernel's DADD by the opcode counters; 24k atoms 567 -> 554 us).
 __device__ __forceinline__ double min_image_bits(double d, double L, double halfL) {
     const long long b = __double_as_longlong(d);
     const bool far = (b & 0x7fffffffffffffffLL) > __double_as_longlong(halfL);
     if (__any_sync(__activemask(), far)) {
-        if (far) d += b < 0 ? L : -L;
+        const double shift = far ? (b < 0 ? L : negated(L)) : 0.0;
+        asm volatile("add.rn.f64 %0, %0, %1;" : "+d"(d) : "d"(shift));
     }
     return d;
 }
