@@ -55,8 +55,11 @@ def _compile(src: str, extra: list[str], hdr: str) -> str:
     if os.path.exists(obj) and os.path.exists(stamp) and open(stamp).read() == key:
         return obj
     # -ffp-contract=off: host FP64 set-up code (box, moduli, influence
-    # function) must round like the reference's unfused x86 build on Arm too
-    cmd = [nvcc()] + ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
+    # function) must round like the reference's unfused x86 build on Arm too;
+    # --compress-mode=none: a module is unpacked when its first kernel is asked
+    # for, which for the FFT's took 15 ms of a process's first context, 1.6 ms
+    # without (the library 8 -> 20 MB)
+    cmd = [nvcc()] + ARCH + ["-O3", "-lineinfo", "--compress-mode=none", "-std=c++17", "-Xcompiler", "-fPIC",
                              "-Xcompiler", "-ffp-contract=off",
                              "-I" + CSRC, "-I" + os.path.join(ROOT, "include")] + extra + ["-c", path, "-o", obj]
     r = subprocess.run(cmd, capture_output=True, text=True)
