@@ -1,6 +1,7 @@
 // Neighbour-list rebuild: cell binning, a deterministic spatial sort of the
-// slots, permutation of the per-atom state, and a full (both directions)
-// per-atom Verlet list built one warp per atom with ballot compaction.
+// slots with the pairing of near atoms that share a list, and the permutation
+// of the per-atom state.  The lists themselves (full, both directions) are
+// built from these by k_build, one warp per pair with ballot compaction.
 //
 // Replaces the reference's per-step std::map voxel hash
 // (core/baseline/src/Forces/NeighborList.cpp:12-154).  The set of pairs that

@@ -1,7 +1,8 @@
 // Neighbour-list build and real-space pair forces on shared-memory tiles.
 //
 // One block per group of consecutive cells (nxm_hood.cuh): the block stages
-// the group's neighbourhood once, then each warp takes atoms of the group.
+// the group's neighbourhood once, then each warp takes pairs of the group's
+// atoms, near ones, which share a list.
 //
 // Physics follows NonbondedForce::DirectForcesAndEnergy
 // (core/baseline/src/Forces/NonbondedForce.cpp:530-585): sigma_ij =
@@ -1118,10 +1119,10 @@ static size_t smem_pairs64(int cap) { return (size_t)cap * sizeof(int4) + tail_b
 // static shared memory of the tile kernels (displacement table and counts)
 constexpr size_t kTileStatic = 25 * kRowCells * sizeof(float4) + 16;
 
-// Two blocks of 16 warps per SM when both blocks' shared memory fits (228 KB
-// per SM, 1 KB reserved per block); otherwise one block of 32 warps, which
-// keeps 32 warps on the SM at the same 64 registers per thread.  (Dense
-// neighbourhoods -- one-cell groups of large cells -- need the latter.)
+// Two blocks per SM when both blocks' shared memory fits (228 KB per SM, 1 KB
+// reserved per block); otherwise one block of twice the warps, which keeps as
+// many on the SM at the same registers per thread.  (Dense neighbourhoods --
+// one-cell groups of large cells -- need the latter.)
 static bool wide(size_t dynamic_smem) { return 2 * (dynamic_smem + kTileStatic + 1024) > 228 * 1024; }
 static int build_warps(int cap) { return wide(smem_build(cap, kHoodWarps)) ? 2 * kHoodWarps : kHoodWarps; }
 
@@ -1234,7 +1235,8 @@ void launch_pairs(const DevView &v, int energy, cudaStream_t st) {
     // neighbourhood for itself: as many blocks as make the busiest SM's share
     // of the atoms least (the pipe that bounds the kernel belongs to the SM,
     // so its time is its atoms, however many blocks hold them).  23,800
-    // atoms, 484 groups on 152 SMs: 652 us with one block per group, 567 so.
+    // atoms, 484 groups on 152 SMs: 652 us with one block per group, 567 so
+    // (554 since, by fewer additions per pair).
     const int per = (v.N + v.ngroups - 1) / v.ngroups;
     int parts = 1, best = 1 << 30;
     for (int p = 1; p <= (per + kWarps64 - 1) / kWarps64; ++p) {

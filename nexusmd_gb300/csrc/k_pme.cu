@@ -1,5 +1,6 @@
-// PME charge spreading and force gathering (B-spline order 5), one thread per
-// atom over all systems of the batch.
+// PME charge spreading and force gathering (B-spline order 5) over all systems
+// of the batch: spread by warps (mixed) or one thread per atom (FP64), gather
+// one thread per atom or, in small systems, five lanes per atom.
 //
 // Grid index and fraction follow InitparticleIndexAndFraction
 // (core/baseline/src/Forces/NonbondedForce.cpp:51-71) in FP64: t = x / L,
