@@ -565,12 +565,27 @@ def workload_config(name, s):
     """The workload as both arms name it: a static description of the system
     and the run parameters (no measured values)."""
     cfg, desc = WORKLOADS[name]
-    list_mb = s.n * 3 * 512 / 1e6  # three 512-byte list chunks per atom at ~560 entries
     return {"workload": desc, "atoms": s.n, "box_nm": float(s.box[0]), "pme_grid": list(s.grid),
             "cutoff_nm": s.cutoff, "ewald_tolerance": s.ewald_tol, "skin_nm": 0.1, "rebuild_interval": 10,
             "dt_fs": DT_PS * 1000, "v0": "Maxwell-Boltzmann 300 K",
             "exceptions": "1-4 pairs scaled 0.8333 Coulomb / 0.5 LJ, 1-2 and 1-3 excluded",
-            "l2": "inputs larger than L2: the neighbour list alone is ~%.0f MB read per step" % list_mb}
+            "l2": "flushed between the timed steps (a buffer of 512 MB written)"}
+
+
+def flushed_steps(eng, steps, device):
+    """Device milliseconds of `steps` steps, each timed by itself behind a
+    write of a buffer larger than the L2 cache: at 94,100 atoms a step reads
+    about 110 MB (the lists 73), which a 129 MB L2 could keep in part."""
+    import torch
+    buf = torch.empty(1 << 29, dtype=torch.uint8, device="cuda:%d" % device)
+    ms = 0.0
+    for k in range(steps):
+        buf.fill_(k & 1)
+        torch.cuda.synchronize(device)
+        ms += eng.time_steps(1, DT_PS)
+    del buf
+    torch.cuda.empty_cache()
+    return ms
 
 
 def ordered(out, tail):
@@ -599,9 +614,13 @@ def native(args):
     barrier(dist)
     rb0 = eng.rebuilds()
     with Clocks(local) as clk:
-        ms = eng.time_steps(args.steps, DT_PS)
+        ms = flushed_steps(eng, args.steps, local)
     ms = allmax(dist, ms)
     rebuilds = eng.rebuilds() - rb0
+    # the same number of further steps in one queue, L2 as a run leaves it
+    warm_rb = eng.rebuilds()
+    warm_ms = eng.time_steps(args.steps, DT_PS)
+    warm_rb = eng.rebuilds() - warm_rb
     launches, rb_launches = eng.launches_per_step()
     per_step = ms / args.steps
     value = replica_throughput(ws, s.n, args.steps, ms * 1e-3)
@@ -619,6 +638,8 @@ def native(args):
 
     out = {"metric": "atom-steps/s", "value": value, "unit": "atom-steps/s", "n_gpus": ws,
            "steps": args.steps, "warmup": args.warmup, "ms_per_step": per_step,
+           "queued_steps": {"ms_per_step": sig(warm_ms / args.steps), "list_rebuilds": warm_rb,
+                            "l2": "not flushed, steps queued one behind another"},
            "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
            "dtype": "f32 forces / i64 fixed-point sums / f64 x,v,E",
            "data": "synthetic (seeded chain + flexible water, shapes of the named config)",
