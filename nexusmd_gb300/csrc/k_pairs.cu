@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(W * 32, W == kHoodWarps ? 2 : 1) k_build(DevVi
 // ------------------------------------------------------------------ pairs
 
 struct PairPrm {
-    float ex2c, a04, k2a, sw, inv_w;  // SysDev::ex2c, a04, k2a; the switching distance, 1 / its width
+    float ex2c, a04, k2a, sw, inv_w;  // SysDev::ex2c, a04, k2a, sw_distf, sw_invf
 };
 
 __device__ __forceinline__ float fast_ex2(float x) {
@@ -546,8 +546,7 @@ __device__ __forceinline__ void near_cutoff(const DevView &v, const SysDev &S, c
     const int2 ab = v.ipair[q];
     const int cnt = min(v.ncount[q].x, c0 + 256);
     const uint16_t *list = pair_list(v, q);
-    const float inv_w = SW && S.use_switch ? 1.0f / (S.cutofff - S.sw_distf) : 0.0f;
-    const PairPrm P{S.ex2c, S.a04, S.k2a, inv_w != 0.0f ? S.sw_distf : 0.0f, inv_w};
+    const PairPrm P{S.ex2c, S.a04, S.k2a, S.sw_distf, S.sw_invf};
     for (int k = c0 + lane; k < cnt; k += 32) {
         const unsigned w = list[list_pos(k)], e = w & 0xfff8u;
         const float4 p = lds128(q_addr + 2 * e);
@@ -651,8 +650,7 @@ __global__ void __launch_bounds__(W * 32, W <= kHoodWarps ? 2 : 1) k_pairs_mixed
     stage<false, true>(v, S, s_q, s_lj, spans, nsp, s_dt);
     const unsigned q_addr = smem_addr(s_q), lj_addr = smem_addr(s_lj);
     const float lo = S.cut2f_lo, cut2 = S.cut2f;
-    const float inv_w = SW && S.use_switch ? 1.0f / (S.cutofff - S.sw_distf) : 0.0f;
-    const PairPrm P{S.ex2c, S.a04, S.k2a, inv_w != 0.0f ? S.sw_distf : 0.0f, inv_w};
+    const PairPrm P{S.ex2c, S.a04, S.k2a, S.sw_distf, S.sw_invf};
     PairSums F;
     F.ec = F.ev = make_float2(0.f, 0.f);
     while (q < q1) {

@@ -69,8 +69,11 @@ enum ErrorBits {
 struct SysDev {
     double lb[3], ub[3], L[3], invL[3], halfL[3];
     double cutoff, cut2, alpha, rlist2, sw_dist;
-    float Lf[3], halfLf[3], cut2f, cut2f_lo, cut2f_hi, alphaf, rlist2f, sw_distf, cutofff;
+    float Lf[3], halfLf[3], cut2f, cut2f_lo, cut2f_hi, alphaf, rlist2f;
+    // the switching function: taken where its distance is below the cutoff;
+    // FP32: the distance and 1 / (cutoff - distance), both 0 where there is none
     int use_switch;
+    float sw_distf, sw_invf;
     int nb_on;                // nonbonded force enabled for this system
     int atom_off, natoms;
     int K[3], Kh;             // PME grid, Kh = K[2]/2 + 1

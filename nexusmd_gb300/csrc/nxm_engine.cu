@@ -660,7 +660,15 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
         D.alpha = H.alpha;
         D.rlist2 = H.rlist * H.rlist;
         D.sw_dist = h.sw_dist;
-        D.use_switch = h.use_switch;
+        // (a distance at or beyond the cutoff, or none that can be compared:
+        // no pair is switched; equal in FP32 only: none in the mixed engine)
+        D.use_switch = h.use_switch && h.sw_dist < h.cutoff ? 1 : 0;
+        {
+            const float rc = (float)h.cutoff, sw = (float)h.sw_dist;
+            const bool on = D.use_switch && sw < rc;
+            D.sw_distf = on ? sw : 0.0f;
+            D.sw_invf = on ? 1.0f / (rc - sw) : 0.0f;
+        }
         D.nb_on = (h.force_mask & NXM_FORCE_NONBONDED) ? 1 : 0;
         D.cut2f = (float)D.cut2;
         D.cut2f_lo = (float)(D.cut2 * (1.0 - 1e-5));
@@ -690,8 +698,6 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
             D.ubkey[d] = dkey(H.ub[d]);
         }
         D.rlist2f = (float)D.rlist2;
-        D.sw_distf = (float)h.sw_dist;
-        D.cutofff = (float)h.cutoff;
         D.atom_off = off;
         D.natoms = h.n;
         D.Kh = H.K[2] / 2 + 1;
