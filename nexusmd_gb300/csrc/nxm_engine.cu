@@ -850,9 +850,10 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
             const SysDev &D = sysd_[s];
             ngr += (size_t)D.nc[0] * D.nc[1] * ((D.nc[2] + group_g[s] - 1) / group_g[s]);
         }
-        const size_t est = (size_t)N_ * (600 + (size_t)pair_stride(stride)) +
-                           (20 + (size_t)pair_stride(stride)) * ((size_t)cell_off + 2) +
-                           ngr * (sizeof(CellGroup) + 4 * (size_t)kGroupSpanWords + 8) +
+        const size_t est = (size_t)N_ * 600 +
+                           ((size_t)pair_first(N_, cell_off) + 1) * (2 * (size_t)pair_stride(stride) + 16) +
+                           12 * ((size_t)cell_off + 2) +
+                           ngr * (sizeof(CellGroup) + 4 * (size_t)kGroupSpanWords + 16) +
                            (size_t)S * (kDtabStride * sizeof(float4) + 24 * E_SLOTS + sizeof(SysDev)) +
                            8 * (size_t)cg_total + 56 * nb + 56 * na + 60 * nt + 88 * nx + 16 * (size_t)roff +
                            24 * (size_t)coff + 24 * (size_t)tw_total + (256u << 10);

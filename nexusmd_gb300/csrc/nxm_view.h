@@ -97,9 +97,12 @@ struct DevView {
 };
 
 // First place in DevView::ipair of the pairs of cell c, whose first slot is
-// `start`: room for (n + 1) / 2 pairs of its n atoms, at most one place of
-// which stays unused.
-__host__ __device__ __forceinline__ int pair_first(int start, int c) { return (start + c) >> 1; }
+// `start`.  A cell of n > 0 atoms raises start + min(start, c) by n + 1 or more
+// (min grows by at least one), so it has room for (n + 1) / 2 pairs; an empty
+// one adds none while no more atoms than cells come before it.  All cells
+// take (atoms + min(atoms, cells)) / 2 places, at most one per atom
+// however large the box; in a filled box at most one place of a cell stays unused.
+__host__ __device__ __forceinline__ int pair_first(int start, int c) { return (start + (start < c ? start : c)) >> 1; }
 
 // Entries a pair's list has room for: the union of any two lists within an
 // atom's capacity, filled up to a multiple of 32; whole 256-entry chunks.
