@@ -10,9 +10,36 @@
 // taken before the update, which is where Engine::Report sits
 // (Engine.cpp:162-188).  The force accumulators are read, converted to FP64
 // and cleared here, so the next step starts from zero without a memset.
+#include <type_traits>
+
 #include "nxm_view.h"
 
 namespace nxm {
+
+// An atom's force words, cleared for the next step.  The FP64 engine keeps the
+// pair kernel's sums apart from the rest until here: they are some hundred
+// single additions per atom, and made onto a bonded force of thousands of
+// kJ/mol/nm each would round at its size (and on their own, split in two, at
+// half as many).  Largest part of the difference to long-precision forces that
+// the order of summation makes, 8,000 charges: 4.0e-16 of the norm with one
+// sum for all, 2.2e-16 so, 1.6e-16 for a sum per lane and a tree.
+template <typename Acc>
+__device__ __forceinline__ void take_forces(const DevView &v, int s, Acc w[3]) {
+    Acc *f[3] = {static_cast<Acc *>(v.fx) + s, static_cast<Acc *>(v.fy) + s, static_cast<Acc *>(v.fz) + s};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        w[c] = *f[c];
+        *f[c] = (Acc)0;
+    }
+    if constexpr (std::is_same<Acc, double>::value) {
+        double2 *a = reinterpret_cast<double2 *>(v.fpair) + 2 * (size_t)s, *b = a + 2 * (size_t)v.N;
+        const double2 a0 = a[0], a1 = a[1], b0 = b[0], b1 = b[1];
+        w[0] += a0.x + b0.x;
+        w[1] += a0.y + b0.y;
+        w[2] += a1.x + b1.x;
+        a[0] = a[1] = b[0] = b[1] = make_double2(0.0, 0.0);
+    }
+}
 
 template <typename Acc>
 __global__ void __launch_bounds__(256) k_integrate(DevView v, double dt, int report) {
@@ -23,13 +50,8 @@ __global__ void __launch_bounds__(256) k_integrate(DevView v, double dt, int rep
     float kef = 0.0f;  // mixed engine (summed as fixed point)
     if (live) {
         const SysDev &S = v.sys[sys];
-        Acc *ax = static_cast<Acc *>(v.fx) + s;
-        Acc *ay = static_cast<Acc *>(v.fy) + s;
-        Acc *az = static_cast<Acc *>(v.fz) + s;
-        const Acc w[3] = {*ax, *ay, *az};
-        *ax = (Acc)0;
-        *ay = (Acc)0;
-        *az = (Acc)0;
+        Acc w[3];
+        take_forces(v, s, w);
         // forces in FP64 where they are needed (reports, FP64 update)
         auto F = [&](int c) { return acc_value(w[c]); };
         double p[3] = {v.x[s], v.y[s], v.z[s]};
@@ -168,15 +190,10 @@ __global__ void k_export(DevView v, int with_forces) {
     v.snap_v[3 * (size_t)o + 1] = v.vy[s];
     v.snap_v[3 * (size_t)o + 2] = v.vz[s];
     if (with_forces) {
-        Acc *ax = static_cast<Acc *>(v.fx) + s;
-        Acc *ay = static_cast<Acc *>(v.fy) + s;
-        Acc *az = static_cast<Acc *>(v.fz) + s;
-        v.snap_f[3 * (size_t)o] = acc_value(*ax);
-        v.snap_f[3 * (size_t)o + 1] = acc_value(*ay);
-        v.snap_f[3 * (size_t)o + 2] = acc_value(*az);
-        *ax = (Acc)0;
-        *ay = (Acc)0;
-        *az = (Acc)0;
+        Acc w[3];
+        take_forces(v, s, w);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v.snap_f[3 * (size_t)o + c] = acc_value(w[c]);
     }
 }
 

@@ -19,6 +19,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "nxm_ewald64.cuh"
 #include "nxm_hood.cuh"
 #include "nxm_view.h"
 
@@ -778,9 +779,9 @@ __global__ void __launch_bounds__(W * 32, W <= kHoodWarps ? 2 : 1) k_pairs_mixed
 //    time, so no lane of an FP64 instruction idles;
 //  * comparisons and conversions, FP64 instructions too, are done on the
 //    numbers' bits;
-//  * 1/r by one third-order step from the FP32 reciprocal root, and the Ewald
-//    terms as erf (an entire function of r^2 over r, Taylor rows in a table
-//    that stays in L1) subtracted from the bare Coulomb term: about 40 FP64
+//  * 1/r by one step from the FP32 reciprocal root (the binomial series of
+//    (1 - e)^(-1/2) to second order), and the Ewald terms from polynomials in
+//    r^2 in a table that stays in L1 (nxm_ewald64.cuh): about 40 FP64
 //    instructions per pair, where erfc, exp, sqrt and the divisions took
 //    about 240 per list entry.  23,800 atoms: 5,390 -> 554 us, the FP64 pipe
 //    busy 79% of the kernel's active cycles; 2,700 atoms: 727 -> 92 us.
@@ -818,12 +819,13 @@ struct Pairs64 {
     const float a2f;
     double fx = 0, fy = 0, fz = 0, ec = 0, ev = 0;
     int cur = -1;  // the atom the warp's sums fx, fy, fz belong to
+    double *sums;  // DevView::fpair: the copy that this lane adds to
 
     __device__ Pairs64(const DevView &v_, const SysDev &S_)
         : v(v_), S(S_), L0(S_.L[0]), L1(S_.L[1]), L2(S_.L[2]), h0(S_.halfL[0]), h1(S_.halfL[1]), h2(S_.halfL[2]),
           cut2(S_.cut2), alpha2(S_.alpha2), alpha3(S_.alpha3), sw_dist(S_.sw_dist),
           sw_inv(SW ? 1.0 / (S_.cutoff - S_.sw_dist) : 0.0), near_bits(bits_of(S_.cut2 * (1.0 - 1e-14))),
-          a2f((float)(S_.alpha2 * kBoysPerUnit)) {}
+          a2f((float)S_.alpha2), sums(v_.fpair + (size_t)4 * v_.N * (threadIdx.x & 1)) {}
 
     // the pair (i, j): j's force by atomics; i's into the warp's sums where i
     // is `cur`, by atomics otherwise
@@ -842,7 +844,7 @@ struct Pairs64 {
         // r^2 to FP32 by its bits (truncated), 1/r from the FP32 estimate y
         // (e = 1 - r^2 y^2 below 2^-20): y (1 + e/2 + 3 e^2 / 8), error e^3
         const int hi = (int)(rb >> 32);
-        const float r2f = __int_as_float(((hi - 0x38000000) << 3) | (int)((unsigned)rb >> 29));
+        float r2f = __int_as_float(((hi - 0x38000000) << 3) | (int)((unsigned)rb >> 29));
         double rinv;
         if (hi > 0x39000000 && hi < 0x46000000) {
             const unsigned yb = __float_as_uint(fast_rsqrt(r2f));
@@ -851,6 +853,7 @@ struct Pairs64 {
             rinv = fma(y * e, fma(e, 0.375, 0.5), y);
         } else {
             rinv = 1.0 / sqrt(r2);  // outside FP32's range (coinciding atoms among them)
+            r2f = (float)r2;
         }
         const double rinv2 = rinv * rinv;
         const double2 li = v.ljd[i], lj = v.ljd[j];
@@ -871,46 +874,28 @@ struct Pairs64 {
                 evdw *= sw;
             }
         }
-        // Ewald: erfc/r^3 + ... = 1/r^3 - alpha^3 H(s); erfc/r = 1/r - alpha E(s)
-        const int row = (int)(r2f * a2f);
-        double coul = 0.0, ecoul = 0.0;
-        if (row < kBoysRows) {
-            const double2 *c = reinterpret_cast<const double2 *>(v.boys) + (kBoysRow / 2) * max(row, 0);
-            const double2 c67 = __ldg(c + 3), c45 = __ldg(c + 2), c23 = __ldg(c + 1), c01 = __ldg(c);
-            const double t = fma(r2, alpha2, -c67.y);
-            double p = fma(c67.x, t, c45.y);
-            p = fma(p, t, c45.x);
-            p = fma(p, t, c23.y);
-            p = fma(p, t, c23.x);
-            p = fma(p, t, c01.y);
-            p = fma(p, t, c01.x);
-            coul = fma(-alpha3, p, rinv * rinv2);
-            if (ENERGY) {
-                const double2 *d = c + (kBoysRow / 2) * kBoysRows;
-                const double2 d67 = __ldg(d + 3), d45 = __ldg(d + 2), d23 = __ldg(d + 1), d01 = __ldg(d);
-                p = fma(d67.x, t, d45.y);
-                p = fma(p, t, d45.x);
-                p = fma(p, t, d23.y);
-                p = fma(p, t, d23.x);
-                p = fma(p, t, d01.y);
-                p = fma(p, t, d01.x);
-                ecoul = fma(-S.alpha, p, rinv);
-            }
-        }
+        // Ewald (nxm_ewald64.cuh); the rows reach past the cutoff, so the
+        // table's end is only for what rounding or a wild r^2 may ask
+        const int row = min(ewald_row(r2f * a2f), v.ewald_rows - 1);
+        const double *c = v.ewald + kEwaldRow * row;
+        const double coul = ewald_term(row, ewald_poly(c, r2, alpha2), alpha3, rinv * rinv2);
+        double ecoul = 0.0;
+        if (ENERGY) ecoul = ewald_term(row, ewald_poly(c + kEwaldRow * v.ewald_rows, r2, alpha2), S.alpha, rinv);
         const double dEdR = fma(qq, coul, vdw * rinv2);
         const double gx = dx * dEdR, gy = dy * dEdR, gz = dz * dEdR;  // on j
-        double *ax = static_cast<double *>(v.fx), *ay = static_cast<double *>(v.fy), *az = static_cast<double *>(v.fz);
-        atomicAdd(ax + j, gx);
-        atomicAdd(ay + j, gy);
-        atomicAdd(az + j, gz);
+        double *fj = sums + 4 * (size_t)j;
+        atomicAdd(fj, gx);
+        atomicAdd(fj + 1, gy);
+        atomicAdd(fj + 2, gz);
         if (i == cur) {
             fx += gx;
             fy += gy;
             fz += gz;
         } else {
-            atomicAdd(ax + i, negated(gx));
-            atomicAdd(ay + i, negated(gy));
-            atomicAdd(az + i, negated(gz));
+            double *fi = sums + 4 * (size_t)i;
+            atomicAdd(fi, negated(gx));
+            atomicAdd(fi + 1, negated(gy));
+            atomicAdd(fi + 2, negated(gz));
         }
         if (ENERGY) {
             ec = fma(qq, ecoul, ec);
@@ -931,8 +916,7 @@ struct Pairs64 {
         c += __shfl_xor_sync(full, c, 4);
         c += __shfl_xor_sync(full, c, 2);
         c += __shfl_xor_sync(full, c, 1);
-        double *f = static_cast<double *>(up8 ? v.fz : (up16 ? v.fy : v.fx));
-        if ((lane & 7) == 0 && lane != 24) atomicAdd(f + cur, negated(c));
+        if ((lane & 7) == 0 && lane != 24) atomicAdd(sums + 4 * (size_t)cur + (up8 ? 2 : (up16 ? 1 : 0)), negated(c));
         fx = fy = fz = 0.0;
     }
 };
@@ -1035,8 +1019,20 @@ __global__ void __launch_bounds__(kWarps64 * 32, 2) k_pairs_fp64(DevView v) {
     }
     __syncwarp();
     if (ENERGY) {
-        energy_add(v.E, G.sys, E_COUL, P.ec);
-        energy_add(v.E, G.sys, E_VDW, P.ev);
+        // one word per block and term: the words' rounding (2^-28 kJ/mol) is
+        // most of these energies' error
+        __shared__ double s_e[2][kWarps64];
+        const double ec = warp_sum(P.ec), ev = warp_sum(P.ev);
+        if (lane == 0) {
+            s_e[0][warp] = ec;
+            s_e[1][warp] = ev;
+        }
+        __syncthreads();
+        if (threadIdx.x < 2) {
+            double e = 0.0;
+            for (int w = 0; w < kWarps64; ++w) e += s_e[threadIdx.x][w];
+            if (e != 0.0) atomic_add_fixed(&v.E[G.sys * E_SLOTS + (threadIdx.x ? E_VDW : E_COUL)], e, kEnergyScale);
+        }
     }
 }
 

@@ -103,12 +103,6 @@ struct SysDev {
     float u2nm[3], cut2f_pre;
 };
 
-// Taylor rows of the FP64 pair kernel's Ewald terms: row k covers s =
-// (alpha r)^2 in [k, k + 1) / kBoysPerUnit; beyond kBoysMax erfc(sqrt s) is
-// below 4e-19, half an ulp of the bare Coulomb term it is a share of.
-constexpr int kBoysPerUnit = 32, kBoysMax = 40, kBoysRows = kBoysPerUnit * kBoysMax;
-constexpr int kBoysRow = 8;  // doubles per row: seven coefficients, the centre
-
 // Flags word layout in device memory.
 struct Flags {
     int error;

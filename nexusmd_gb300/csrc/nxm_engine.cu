@@ -23,6 +23,7 @@
 #include <tuple>
 
 #include "nxm_engine.h"
+#include "nxm_ewald64.cuh"
 
 namespace nxm {
 
@@ -214,45 +215,6 @@ static void bspline_moduli(int K, std::vector<double> &mod) {
 // buffer, then a merge with the atom's sorted exception partners.  The
 // creation builds the same sets on the device (k_exclusions_build.cu); this
 // host form serves a batch with a row longer than the device search holds.
-// Taylor rows of the FP64 pair kernel's Ewald terms (nxm_common.cuh:
-// kBoysRows), made once per process.  With s = (alpha r)^2,
-//   erf(alpha r) / (alpha r)                                = 2/sqrt(pi) F_0(s)
-//   (erf(alpha r) - 2 alpha r e^-s / sqrt(pi)) / (alpha r)^3 = 4/sqrt(pi) F_1(s)
-// where F_m(s) = integral_0^1 t^2m e^(-s t^2) dt (the Boys functions), and
-// dF_m/ds = -F_(m+1) gives the coefficients about a row's centre: degree 6
-// over half a row (1/64) leaves (1/64)^7 / 7! / 17 < 1e-17.  F_m comes from
-// its series at the highest order, whose terms are all positive, and from
-// there by downward recursion, which is stable: each value within a few ulp.
-static const std::vector<double> &boys_rows() {
-    static const std::vector<double> rows = [] {
-        std::vector<double> t((size_t)2 * kBoysRows * kBoysRow);
-        for (int k = 0; k < kBoysRows; ++k) {
-            const double s = (k + 0.5) / kBoysPerUnit, ex = std::exp(-s);
-            constexpr int M = kBoysRow - 1;
-            double F[M + 1];
-            double term = 1.0 / (2 * M + 1), sum = term;
-            for (int j = 1; term > sum * 1e-18; ++j) {
-                term *= 2 * s / (2 * M + 2 * j + 1);
-                sum += term;
-            }
-            F[M] = ex * sum;
-            for (int m = M - 1; m >= 0; --m) F[m] = (2 * s * F[m + 1] + ex) / (2 * m + 1);
-            for (int which = 0; which < 2; ++which) {
-                // which 0: the force's rows (F_1), 1: the energy's (F_0)
-                double *row = &t[((size_t)which * kBoysRows + k) * kBoysRow];
-                double f = (which ? 2.0 : 4.0) / kSqrtPi;
-                for (int c = 0; c < kBoysRow - 1; ++c) {
-                    row[c] = f * F[c + (which ? 0 : 1)];
-                    f /= -(c + 1);
-                }
-                row[kBoysRow - 1] = s;
-            }
-        }
-        return t;
-    }();
-    return rows;
-}
-
 static std::string exclusion_rows(const HostSystem &s, int off, std::vector<int> &eoff, std::vector<int> &elst,
                                   std::vector<int2> &ex_pairs) {
     const int n = s.n;
@@ -678,7 +640,7 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
         D.a04 = (float)(0.4 * H.alpha);
         D.k2a = (float)(2.0 * H.alpha / kSqrtPi);
         D.alpha2 = H.alpha * H.alpha;
-        D.alpha3 = D.alpha2 * H.alpha;
+        D.alpha3 = (double)((long double)H.alpha * H.alpha * H.alpha);  // rounded once
         {
             // relative rounding of the filter's FP32 r^2 (< 1e-6) and its
             // grain: each displacement is within 2 units of 2^-32 of the edge
@@ -838,7 +800,7 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
         // one reservation for the context's device arrays (an upper
         // estimate; a shortfall comes out of further chunks): per atom the
         // state, derived inputs, cell keys, exclusion build, PME stencils,
-        // snapshots and frames (~600 B) and the list; per cell, group, term,
+        // snapshots and frames (~600 B, FP64 100 more) and the list; per cell, group, term,
         // exception and grid point their tables
         size_t nb = 0, na = 0, nt = 0, nx = 0, ngr = 0;
         for (int s = 0; s < S; ++s) {
@@ -850,7 +812,7 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
             const SysDev &D = sysd_[s];
             ngr += (size_t)D.nc[0] * D.nc[1] * ((D.nc[2] + group_g[s] - 1) / group_g[s]);
         }
-        const size_t est = (size_t)N_ * 600 +
+        const size_t est = (size_t)N_ * (mixed_ ? 600 : 700) +
                            ((size_t)pair_first(N_, cell_off) + 1) * (2 * (size_t)pair_stride(stride) + 16) +
                            12 * ((size_t)cell_off + 2) +
                            ngr * (sizeof(CellGroup) + 4 * (size_t)kGroupSpanWords + 16) +
@@ -880,6 +842,7 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
         v_.fx = dalloc<double>(N_);
         v_.fy = dalloc<double>(N_);
         v_.fz = dalloc<double>(N_);
+        v_.fpair = dalloc<double>(8 * (size_t)N_);
     }
     v_.cell3 = dalloc<int>(N_);
     v_.total_cells = cell_off;
@@ -968,12 +931,15 @@ std::string Engine::init(const std::vector<HostSystem> &systems, const nxm_optio
     up(v_.tmp, positions, sizeof(double) * 3 * (size_t)N_);
     launch_init_atoms(v_, v_.tmp, kst());
 
-    double *boys = nullptr;
     if (!mixed_) {
-        const std::vector<double> &t = boys_rows();
-        boys = dalloc<double>(t.size());
-        up(boys, t.data(), sizeof(double) * t.size());
-        v_.boys = boys;
+        double smax = 0.0;
+        for (const SysDev &D : sysd_)
+            if (D.nb_on) smax = std::max(smax, D.cut2 * D.alpha2);
+        std::vector<double> rows;
+        v_.ewald_rows = ewald_rows(smax, rows);
+        double *d = dalloc<double>(rows.size());
+        up(d, rows.data(), sizeof(double) * rows.size());
+        v_.ewald = d;
     }
 
     // cell-image displacement table: code ((ox+2)*5 + (oy+2))*12 + (oz+2) -> -(o . cs),

@@ -37,10 +37,12 @@ struct DevView {
     double *qs;          // fp64: q * sqrt(ke)
     double2 *ljd;        // fp64: sigma/2, 2 sqrt(eps)
     int4 *uf;            // fp64: box fraction (p - lb) / L of x, y, z modulo 1, in 2^-32 (the pair kernel's filter)
-    const double *boys;  // fp64: Taylor rows of the Ewald terms: [kBoysRows][kBoysRow] force, then energy
+    const double *ewald; // fp64: polynomials of the Ewald terms (nxm_ewald64.cuh): [ewald_rows][kEwaldRow] force, then energy
+    int ewald_rows;
     int *cell3;          // slot -> packed cell coordinates (x | y<<10 | z<<20)
     // force accumulators (long long in mixed mode, double in fp64 mode)
     void *fx, *fy, *fz;
+    double *fpair;       // fp64: [2][N][4] sums of the pair kernel's forces x, y, z, apart from the others' (take_forces)
     // neighbour list
     int total_cells;
     int *cell_key, *cell_count, *cell_start, *cell_fill;
