@@ -480,9 +480,10 @@ __device__ __forceinline__ float2 erfcx_fit2(float2 t) {
 // both, NonbondedForce.cpp:559-581 in single precision, in the two halves of
 // packed FP32x2 operations (one instruction for both; the reciprocal square
 // root, exponential and reciprocal are scalar), added to the lane's sums
-// where `in`.  Without branches: an entry outside the cutoff gives finite
-// values that a select drops (with energies: selects on the charge product
-// and epsilon, which every term has as a factor; four selects for six).
+// where `in`.  Without branches: an entry outside the cutoff (or at a distance
+// that is not a number) gives a value that a select drops.  The selects are on
+// the results: a factor set to zero instead would still carry a NaN into the
+// sums.
 // exp(-(alpha r)^2) comes straight from r^2; erfc(alpha r) =
 // exp(-(alpha r)^2) g(t), t = 1 / (1 + 0.4 alpha r).
 struct PairSums {
@@ -492,10 +493,7 @@ struct PairSums {
 template <bool ENERGY, bool SW>
 __device__ __forceinline__ void pair_mixed2(bool in0, bool in1, float2 dx, float2 dy, float2 dz, float2 r2, float2 qq,
                                             float2 sg, float2 eps, const PairPrm &P, PairSums &F) {
-    if (ENERGY) {
-        qq = make_float2(in0 ? qq.x : 0.0f, in1 ? qq.y : 0.0f);
-        eps = make_float2(in0 ? eps.x : 0.0f, in1 ? eps.y : 0.0f);
-    }
+    auto only = [&](float2 a) { return make_float2(in0 ? a.x : 0.0f, in1 ? a.y : 0.0f); };
     const float2 rinv = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
     const float2 rinv2 = __fmul2_rn(rinv, rinv);
     const float2 r = __fmul2_rn(r2, rinv);
@@ -505,7 +503,7 @@ __device__ __forceinline__ void pair_mixed2(bool in0, bool in1, float2 dx, float
     const float2 erfcv = __fmul2_rn(ex, erfcx_fit2(make_float2(fast_rcp(tt.x), fast_rcp(tt.y))));
     const float2 qr = __fmul2_rn(qq, rinv);
     float2 dEdR = __fmul2_rn(__fmul2_rn(qr, rinv2), __ffma2_rn(__fmul2_rn(dup2(P.k2a), r), ex, erfcv));
-    if (ENERGY) F.ec = __ffma2_rn(qr, erfcv, F.ec);
+    if (ENERGY) F.ec = __fadd2_rn(F.ec, only(__fmul2_rn(qr, erfcv)));
     const float2 s2 = __fmul2_rn(__fmul2_rn(sg, sg), rinv2);
     const float2 s6 = __fmul2_rn(__fmul2_rn(s2, s2), s2);
     const float2 es6 = __fmul2_rn(eps, s6);
@@ -523,12 +521,11 @@ __device__ __forceinline__ void pair_mixed2(bool in0, bool in1, float2 dx, float
                                        __ffma2_rn(t, __ffma2_rn(t, dup2(30.0f), dup2(-60.0f)), dup2(30.0f)));
         const float2 l = __ffma2_rn(es6, s6, make_float2(-es6.x, -es6.y));
         lj = __ffma2_rn(sw, lj, __fmul2_rn(__fmul2_rn(l, mdsw), r));
-        if (ENERGY) F.ev = __ffma2_rn(l, sw, F.ev);
+        if (ENERGY) F.ev = __fadd2_rn(F.ev, only(__fmul2_rn(l, sw)));
     } else if (ENERGY) {
-        F.ev = __fadd2_rn(F.ev, __ffma2_rn(es6, s6, make_float2(-es6.x, -es6.y)));
+        F.ev = __fadd2_rn(F.ev, only(__ffma2_rn(es6, s6, make_float2(-es6.x, -es6.y))));
     }
-    dEdR = __ffma2_rn(lj, rinv2, dEdR);
-    if (!ENERGY) dEdR = make_float2(in0 ? dEdR.x : 0.0f, in1 ? dEdR.y : 0.0f);
+    dEdR = only(__ffma2_rn(lj, rinv2, dEdR));
     F.fx = __ffma2_rn(dx, dEdR, F.fx);
     F.fy = __ffma2_rn(dy, dEdR, F.fy);
     F.fz = __ffma2_rn(dz, dEdR, F.fz);
