@@ -1,8 +1,8 @@
 """Builds libnxm_cuda.so in the package directory with nvcc for sm_103a.
 
 Each translation unit is compiled separately (in parallel) into _build/,
-then linked into nexusmd_gb300/libnxm_cuda.so.  Only files whose sources or
-headers changed are recompiled.  Host-only C++ goes through nvcc too, so the
+then linked into nexusmd_gb300/libnxm_cuda.so.  Only files whose sources,
+headers or compile command changed are recompiled.  Host-only C++ goes through nvcc too, so the
 same compiler and flags are used on x86 and on Arm hosts.
 """
 from __future__ import annotations
@@ -46,22 +46,39 @@ def _headers_digest() -> str:
     return h.hexdigest()
 
 
-def _compile(src: str, extra: list[str], hdr: str) -> str:
-    path = os.path.join(CSRC, src)
-    obj = os.path.join(BUILD, src + ".o")
-    stamp = obj + ".stamp"
-    with open(path, "rb") as f:
-        key = hashlib.sha256(f.read() + hdr.encode() + " ".join(extra).encode()).hexdigest()
-    if os.path.exists(obj) and os.path.exists(stamp) and open(stamp).read() == key:
-        return obj
+def _compiler_version() -> str:
+    return subprocess.run([nvcc(), "--version"], capture_output=True, text=True).stdout
+
+
+def _command(src: str, extra: list[str], obj: str) -> list[str]:
     # -ffp-contract=off: host FP64 set-up code (box, moduli, influence
     # function) must round like the reference's unfused x86 build on Arm too;
     # --compress-mode=none: a module is unpacked when its first kernel is asked
     # for, which for the FFT's took 15 ms of a process's first context, 1.6 ms
     # without (the library 8 -> 20 MB)
-    cmd = [nvcc()] + ARCH + ["-O3", "-lineinfo", "--compress-mode=none", "-std=c++17", "-Xcompiler", "-fPIC",
-                             "-Xcompiler", "-ffp-contract=off",
-                             "-I" + CSRC, "-I" + os.path.join(ROOT, "include")] + extra + ["-c", path, "-o", obj]
+    return ([nvcc()] + ARCH + ["-O3", "-lineinfo", "--compress-mode=none", "-std=c++17", "-Xcompiler", "-fPIC",
+                               "-Xcompiler", "-ffp-contract=off",
+                               "-I" + CSRC, "-I" + os.path.join(ROOT, "include")]
+            + extra + ["-c", os.path.join(CSRC, src), "-o", obj])
+
+
+def _key(cmd: list[str], source: str, *rest: str) -> str:
+    """What an output depends on: the command (flags, paths), the compiler,
+    the source and the rest (headers)."""
+    h = hashlib.sha256("\0".join(cmd + list(rest)).encode())
+    with open(source, "rb") as f:
+        h.update(f.read())
+    return h.hexdigest()
+
+
+def _compile(src: str, extra: list[str], hdr: str, version: str) -> str:
+    path = os.path.join(CSRC, src)
+    obj = os.path.join(BUILD, src + ".o")
+    stamp = obj + ".stamp"
+    cmd = _command(src, extra, obj)
+    key = _key(cmd, path, hdr, version)
+    if os.path.exists(obj) and os.path.exists(stamp) and open(stamp).read() == key:
+        return obj
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("nvcc failed for %s:\n%s\n%s" % (src, " ".join(cmd), r.stderr[-8000:]))
@@ -73,11 +90,11 @@ def _compile(src: str, extra: list[str], hdr: str) -> str:
 def build(verbose: bool = False) -> str:
     """Compile and link; returns the library path."""
     os.makedirs(BUILD, exist_ok=True)
-    hdr = _headers_digest()
+    hdr, version = _headers_digest(), _compiler_version()
     jobs = [(s, ["-x", "cu"] if s.endswith(".cpp") else []) for s in CUDA_SOURCES]
     jobs += [(s, ["-x", "c++"]) for s in HOST_SOURCES if os.path.exists(os.path.join(CSRC, s))]
     with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 4)) as ex:
-        objs = list(ex.map(lambda j: _compile(j[0], j[1], hdr), jobs))
+        objs = list(ex.map(lambda j: _compile(j[0], j[1], hdr, version), jobs))
     tmp = LIB + ".tmp"
     cmd = [nvcc()] + ARCH + ["-shared", "-o", tmp] + objs + ["-lcudart"]
     r = subprocess.run(cmd, capture_output=True, text=True)
@@ -94,13 +111,12 @@ def build_probe(verbose: bool = False) -> str:
     """Compile bench_probe.cu into libnxm_probe.so (bench.py's hardware probes)."""
     os.makedirs(BUILD, exist_ok=True)
     stamp = os.path.join(BUILD, "probe.stamp")
-    with open(PROBE_SRC, "rb") as f:
-        key = hashlib.sha256(f.read()).hexdigest()
-    if os.path.exists(PROBE_LIB) and os.path.exists(stamp) and open(stamp).read() == key:
-        return PROBE_LIB
     tmp = PROBE_LIB + ".tmp"
     cmd = [nvcc()] + ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-shared",
                              PROBE_SRC, "-o", tmp]
+    key = _key(cmd, PROBE_SRC, _compiler_version())
+    if os.path.exists(PROBE_LIB) and os.path.exists(stamp) and open(stamp).read() == key:
+        return PROBE_LIB
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("nvcc failed for bench_probe.cu:\n" + r.stderr[-4000:])
