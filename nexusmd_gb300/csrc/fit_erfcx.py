@@ -7,7 +7,7 @@ so a degree-6 polynomial in t, least-squares fitted on Chebyshev nodes of t
 (a near-minimax fit), holds g to ~3e-7 relative in exact arithmetic and
 ~5e-7 when evaluated by Horner's rule in FP32 (degree 8: 1e-8 and 2.5e-7,
 two more multiply-adds per pair for no gain that FP32 keeps).  Run this
-file to print the coefficients pasted into nxm_common.cuh.
+file to print the coefficients pasted into k_pairs.cu (erfcx_fit2).
 """
 import numpy as np
 from scipy.special import erfcx

@@ -465,6 +465,10 @@ __device__ __forceinline__ float fast_ex2(float x) {
 
 __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 
+// g(t) of erfc(x) = exp(-x^2) g(t), t = 1 / (1 + 0.4 x), x in [0, 4]: degree-6
+// least-squares fit of the scaled complementary error function on Chebyshev
+// nodes of t, max relative error 5e-7 in FP32 (derivation and error table:
+// fit_erfcx.py next to this file).
 __device__ __forceinline__ float2 erfcx_fit2(float2 t) {
     float2 g = dup2(-2.164941738e-01f);
     g = __ffma2_rn(g, t, dup2(7.803782561e-01f));
@@ -531,12 +535,18 @@ __device__ __forceinline__ void pair_mixed2(bool in0, bool in1, float2 dx, float
     F.fz = __ffma2_rn(dz, dEdR, F.fz);
 }
 
+// Whether list entry w, at an FP32 r^2 from atom m of its pair (0 the first, 1
+// the second), is too near the cutoff for FP32 to tell: within 1e-5, and not
+// excluded.  Then exact_r2 decides as the reference does.
+__device__ __forceinline__ bool at_cutoff(const SysDev &S, unsigned w, int m, float r2) {
+    return !((w >> m) & 1) && r2 >= S.cut2f_lo && r2 < S.cut2f_hi;
+}
+
 // The entries of one chunk (c0) of pair q's list whose FP32 r^2 is within
-// 1e-5 of the cutoff's, which the walk left out: decided in FP64 exactly as
-// the reference, and added where they are within it.  One chunk in a hundred
-// comes here.  The energies' kernel calls it when the pair is done, with its
-// own atomics, so that its registers are not added to the walk's (179 -> 157
-// us at 94,100 atoms).
+// 1e-5 of the cutoff's, which the walk left out: decided in FP64 (at_cutoff) and
+// added where they are within it.  One chunk in a hundred comes here.  The energies'
+// kernel calls it when the pair is done, with its own atomics, so that its
+// registers are not added to the walk's (179 -> 157 us at 94,100 atoms).
 template <bool ENERGY, bool SW>
 __device__ __forceinline__ void near_cutoff(const DevView &v, const SysDev &S, const HoodSpan *spans, int nsp, int kbase,
                                             int q, int c0, unsigned q_addr, unsigned lj_addr) {
@@ -551,11 +561,11 @@ __device__ __forceinline__ void near_cutoff(const DevView &v, const SysDev &S, c
         const float2 l = lds64(lj_addr + e);
         for (int m = 0; m < 2; ++m) {
             const int i = m ? ab.y : ab.x;
-            if (i < 0 || ((w >> m) & 1)) continue;
+            if (i < 0) continue;
             const float4 pi = lds128(q_addr + 16 * (kbase + i));
             const float dx = pi.x - p.x, dy = pi.y - p.y, dz = pi.z - p.z;
             const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-            if (!(r2 >= S.cut2f_lo && r2 < S.cut2f_hi)) continue;
+            if (!at_cutoff(S, w, m, r2)) continue;
             if (!(exact_r2(v, S, i, hood_slot(spans, nsp, (int)(e >> kEntryShift))) < S.cut2)) continue;
             const float2 li = lds64(lj_addr + 8 * (kbase + i));
             PairSums F;
@@ -722,8 +732,7 @@ __global__ void __launch_bounds__(W * 32, W <= kHoodWarps ? 2 : 1) k_pairs_mixed
                         const float2 dy = make_float2(pa.y - p.y, pb.y - p.y);
                         const float2 dz = make_float2(pa.z - p.z, pb.z - p.z);
                         const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-                        bool in0 = !(w & 1) && r2.x >= lo && r2.x < S.cut2f_hi;
-                        bool in1 = !(w & 2) && r2.y >= lo && r2.y < S.cut2f_hi;
+                        bool in0 = at_cutoff(S, w, 0, r2.x), in1 = at_cutoff(S, w, 1, r2.y);
                         if (!(in0 || in1)) continue;
                         const int j = hood_slot(spans, nsp, (int)(e >> kEntryShift));
                         in0 = in0 && exact_r2(v, S, ab.x, j) < S.cut2;

@@ -295,21 +295,6 @@ __device__ __forceinline__ void energy_add_fixed(long long *E, int sys, int term
         atomicAdd(reinterpret_cast<unsigned long long *>(&E[sys * E_SLOTS + term]), static_cast<unsigned long long>(v));
 }
 
-// erfc(x) = exp(-x^2) * g(t), t = 1 / (1 + 0.4 x), x in [0, 4]: degree-6
-// least-squares fit of the scaled complementary error function on Chebyshev
-// nodes of t, max relative error 5e-7 in FP32 (derivation and error table:
-// fit_erfcx.py next to this file).
-__device__ __forceinline__ float erfcx_fit(float t) {
-    float g = -2.164941738e-01f;
-    g = fmaf(g, t, 7.803782561e-01f);
-    g = fmaf(g, t, -4.985805536e-01f);
-    g = fmaf(g, t, 5.875147125e-01f);
-    g = fmaf(g, t, 1.009222009e-01f);
-    g = fmaf(g, t, 2.479314205e-01f);
-    g = fmaf(g, t, -1.671998421e-03f);
-    return g;
-}
-
 __device__ __forceinline__ float fast_rcp(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
