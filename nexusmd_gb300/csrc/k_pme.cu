@@ -41,7 +41,9 @@ __global__ void __launch_bounds__(256) k_spread(DevView v, const FftSysDev *fs) 
         t = (t - floor(t)) * F.K[d];
         int ti = (int)t;
         fr[d] = (R)(t - ti);
-        idx[d] = ti % F.K[d];
+        // (a coordinate that is not finite converts to the least integer,
+        // whose remainder would be an index below the grid)
+        idx[d] = ti > 0 ? ti % F.K[d] : 0;
     }
     v.pme_idx[s] = make_int4(idx[0], idx[1], idx[2], 0);
     if (sizeof(R) == 4) {

@@ -89,7 +89,7 @@ __device__ __forceinline__ void grid_coord(double p, double invL, int K, int &id
     t = (t - floor(t)) * K;
     int ti = (int)t;
     fr = (float)(t - ti);
-    idx = ti % K;
+    idx = ti > 0 ? ti % K : 0;  // (not finite: the least integer)
 }
 
 // |b(k)|^2 of one axis: the order-5 spline's values at the integers are
