@@ -25,12 +25,16 @@ namespace nxm {
 // sum for all, 2.2e-16 so, 1.6e-16 for a sum per lane and a tree.
 template <typename Acc>
 __device__ __forceinline__ void take_forces(const DevView &v, int s, Acc w[3]) {
-    Acc *f[3] = {static_cast<Acc *>(v.fx) + s, static_cast<Acc *>(v.fy) + s, static_cast<Acc *>(v.fz) + s};
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        w[c] = *f[c];
-        *f[c] = (Acc)0;
-    }
+    Acc *ax = static_cast<Acc *>(v.fx) + s;
+    Acc *ay = static_cast<Acc *>(v.fy) + s;
+    Acc *az = static_cast<Acc *>(v.fz) + s;
+    // (all loads before the first store, which might alias them)
+    w[0] = *ax;
+    w[1] = *ay;
+    w[2] = *az;
+    *ax = (Acc)0;
+    *ay = (Acc)0;
+    *az = (Acc)0;
     if constexpr (std::is_same<Acc, double>::value) {
         double2 *a = reinterpret_cast<double2 *>(v.fpair) + 2 * (size_t)s, *b = a + 2 * (size_t)v.N;
         const double2 a0 = a[0], a1 = a[1], b0 = b[0], b1 = b[1];

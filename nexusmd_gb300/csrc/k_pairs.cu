@@ -538,8 +538,9 @@ __device__ __forceinline__ void pair_mixed2(bool in0, bool in1, float2 dx, float
 // Whether list entry w, at an FP32 r^2 from atom m of its pair (0 the first, 1
 // the second), is too near the cutoff for FP32 to tell: within 1e-5, and not
 // excluded.  Then exact_r2 decides as the reference does.
-__device__ __forceinline__ bool at_cutoff(const SysDev &S, unsigned w, int m, float r2) {
-    return !((w >> m) & 1) && r2 >= S.cut2f_lo && r2 < S.cut2f_hi;
+// (lo: S.cut2f_lo, which the walk holds in a register)
+__device__ __forceinline__ bool at_cutoff(const SysDev &S, unsigned w, unsigned m, float r2, float lo) {
+    return !(w & (1u << m)) && r2 >= lo && r2 < S.cut2f_hi;
 }
 
 // The entries of one chunk (c0) of pair q's list whose FP32 r^2 is within
@@ -565,7 +566,7 @@ __device__ __forceinline__ void near_cutoff(const DevView &v, const SysDev &S, c
             const float4 pi = lds128(q_addr + 16 * (kbase + i));
             const float dx = pi.x - p.x, dy = pi.y - p.y, dz = pi.z - p.z;
             const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-            if (!at_cutoff(S, w, m, r2)) continue;
+            if (!at_cutoff(S, w, m, r2, S.cut2f_lo)) continue;
             if (!(exact_r2(v, S, i, hood_slot(spans, nsp, (int)(e >> kEntryShift))) < S.cut2)) continue;
             const float2 li = lds64(lj_addr + 8 * (kbase + i));
             PairSums F;
@@ -732,7 +733,8 @@ __global__ void __launch_bounds__(W * 32, W <= kHoodWarps ? 2 : 1) k_pairs_mixed
                         const float2 dy = make_float2(pa.y - p.y, pb.y - p.y);
                         const float2 dz = make_float2(pa.z - p.z, pb.z - p.z);
                         const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-                        bool in0 = at_cutoff(S, w, 0, r2.x), in1 = at_cutoff(S, w, 1, r2.y);
+                        bool in0 = at_cutoff(S, w, 0, r2.x, lo);
+                        bool in1 = at_cutoff(S, w, 1, r2.y, lo);
                         if (!(in0 || in1)) continue;
                         const int j = hood_slot(spans, nsp, (int)(e >> kEntryShift));
                         in0 = in0 && exact_r2(v, S, ab.x, j) < S.cut2;
