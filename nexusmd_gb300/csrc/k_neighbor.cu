@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_cellsort(DevView v) {
     __shared__ float s_pos[kSortWarps][3][kSortMax];
     const unsigned full = 0xffffffffu;
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int c = blockIdx.x * (blockDim.x >> 5) + warp;
+    int c = blockIdx.x * kSortWarps + warp;
     if (c >= v.total_cells) return;
     int a = v.cell_start[c], n = v.cell_start[c + 1] - a;
     // the cell's count and fill words, done with, start the next rebuild at zero
@@ -344,11 +344,10 @@ void launch_remap_terms(const DevView &v, cudaStream_t st) {
 
 void launch_nlist_order(const DevView &v, cudaStream_t st) {
     const int t = thread_block(v.N);
-    const int w = v.total_cells >= 2 * 152 * kSortWarps ? kSortWarps : 1;
     k_assign<<<blocks(v.N, t), t, 0, st>>>(v);
     k_scan<<<1, 1024, 0, st>>>(v.flags, v.cell_count, v.cell_start, v.total_cells);
     k_scatter<<<blocks(v.N, t), t, 0, st>>>(v);
-    k_cellsort<<<blocks(v.total_cells, w), w * 32, 0, st>>>(v);
+    k_cellsort<<<blocks(v.total_cells, kSortWarps), kSortWarps * 32, 0, st>>>(v);
     k_permute_gather<<<blocks(v.N, t), t, 0, st>>>(v);
     k_permute_scatter<<<blocks(v.N, t), t, 0, st>>>(v);
     long long nt = (long long)v.nb + v.na + v.nt + v.nex + v.nxc;

@@ -1242,7 +1242,7 @@ void launch_pairs(const DevView &v, int energy, cudaStream_t st) {
     const int per = (v.N + v.ngroups - 1) / v.ngroups;
     int parts = 1, best = 1 << 30;
     for (int p = 1; p <= (per + kWarps64 - 1) / kWarps64; ++p) {
-        const long long rounds = ((long long)v.ngroups * p + 151) / 152;
+        const long long rounds = ((long long)v.ngroups * p + kSMs - 1) / kSMs;
         const int cost = (int)std::min<long long>(rounds * ((per + p - 1) / p), 1 << 29);
         if (cost <= best) {
             best = cost;

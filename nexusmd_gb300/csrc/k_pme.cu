@@ -225,10 +225,11 @@ __global__ void __launch_bounds__(256) k_gather(DevView v, const FftSysDev *fs) 
 // The gather of the mixed engine with five lanes per atom, one x-plane of the
 // stencil each, six atoms per warp: a fifth of the loads in a thread's chain.
 // For systems too small to give every SM a block of a thread per atom, where
-// that chain is the kernel's time: 2,700 atoms 10.2 -> 8.2 us.  With more the
-// threads hide it and the repeated weights cost more: 23,800 atoms 12.0 us
-// with a thread per atom, 14.3 so; 94,100: 16.4 and 20.5.
-constexpr int kPlaneThreads = 64, kPlaneAtoms = 152 * 64;
+// that chain is the kernel's time: 2,700 and 5,400 atoms 10.2 -> 8.2 us.  With
+// more the threads hide it and the repeated weights cost more: 8,100 atoms 10.4
+// us with a thread per atom, 10.2 so; 10,800: 10.3 and 10.2; 16,200: 10.9 and
+// 12.3; 23,800: 12.0 and 14.3; 94,100: 16.4 and 20.5.
+constexpr int kPlaneThreads = 64, kPlaneAtoms = 64 * kSMs;
 
 __global__ void __launch_bounds__(kPlaneThreads) k_gather_planes(DevView v, const FftSysDev *fs) {
     const unsigned full = 0xffffffffu;
@@ -323,12 +324,16 @@ void launch_clear_grid(const DevView &v, cudaStream_t st) {
 void launch_spread(const DevView &v, const FftPlan &plan, cudaStream_t st) {
     int t = v.pme_block, nb = (v.N + t - 1) / t;
     if (v.mixed) {
-        // 16 atoms per warp, fewer where that leaves SMs idle: a warp takes
-        // its atoms one after the other
+        // 16 atoms per warp, fewer where those warps would not fill the SMs: a
+        // warp takes its atoms one after the other.  With 4, 8 and 16 per warp:
+        // 2,700 atoms 10.7, 10.7, 13.7 us; 10,800 12.8, 12.9, 13.8; 16,200 13.8,
+        // 13.8, 14.4; 23,800 15.3, 15.2, 17.3; 48,600 21.8, 20.1, 22.3; 64,800
+        // 25.7, 25.2, 26.7; 97,200 (8, 16) 31.4, 31.3, the step 263, 269; 145,800
+        // 39.4, 39.4; 259,200 64, 64, the step 636, 629.
         auto grid = [&](int atoms) { return (v.N + kSpreadWarps * atoms - 1) / (kSpreadWarps * atoms); };
-        if (grid(16) >= 2 * 152)
+        if (grid(16) >= 6 * kSMs)
             k_spread_warp<16><<<grid(16), kSpreadWarps * 32, 0, st>>>(v, plan.dsys);
-        else if (grid(8) >= 152)
+        else if (grid(8) >= kSMs)
             k_spread_warp<8><<<grid(8), kSpreadWarps * 32, 0, st>>>(v, plan.dsys);
         else
             k_spread_warp<4><<<grid(4), kSpreadWarps * 32, 0, st>>>(v, plan.dsys);

@@ -355,9 +355,9 @@ extern "C" int nxm_pme_reciprocal_noalloc(const double *xyz, const double *charg
     if (pending != cudaSuccess)
         return fail(NXM_ERR_CUDA, std::string(fn) + "a CUDA error was already pending: " +
                                       cudaGetErrorString(pending));
-    k_noalloc_setup<<<kAxisBlocks + 152, 256, 0, st>>>(scr, g);
+    k_noalloc_setup<<<kAxisBlocks + kSMs, 256, 0, st>>>(scr, g);
     const int nspread = (n_atoms + kSpreadBlockWarps * kAtoms - 1) / (kSpreadBlockWarps * kAtoms);
-    const int neterm = (int)std::min<long long>((v.total_cgrid + kSpreadBlockWarps * 32 - 1) / (kSpreadBlockWarps * 32), 608);
+    const int neterm = (int)std::min<long long>((v.total_cgrid + kSpreadBlockWarps * 32 - 1) / (kSpreadBlockWarps * 32), 4 * kSMs);
     // (the first kernel is an ordinary launch: it follows whatever the caller
     // put on the stream)
     plan.chained = true;

@@ -30,6 +30,7 @@ constexpr double kGridUnscale = 1.0 / 16777216.0;
 constexpr double kEnergyScale = 268435456.0;
 constexpr double kEnergyUnscale = 1.0 / 268435456.0;
 
+constexpr int kSMs = 152;      // of a GB300, for which this is built: the launch rules count blocks per SM by it
 constexpr int kOrder = 5;       // PME B-spline order (NonbondedForce.cpp:474)
 constexpr int kCodeBits = 7;    // list entry = slot (25 bits) | cell-image code (7 bits)
 constexpr uint32_t kSlotMask = (1u << 25) - 1u;

@@ -1544,7 +1544,8 @@ std::string Engine::build_graph(double dt, int report) {
     return r;
 }
 
-constexpr int kSplitAtoms = 10000;
+// From here on the lists have a conditional node of their own (build_graph_timed).
+constexpr int kSplitAtoms = 64000;
 
 std::string Engine::build_graph_timed(double dt, int report) {
     StepGraph &G = graph_[report];
@@ -1608,10 +1609,12 @@ std::string Engine::build_graph_timed(double dt, int report) {
     // new slot order, when the decision asks for one; behind it the PME chain
     // on a branch of its own, and on the other the lists (when asked for), the
     // bonded terms and the pairs; the update behind both.  The PME chain needs
-    // no lists, so on a step that rebuilds it runs beside their build: 20 steps
-    // at 94,100 atoms 5.46 -> 5.33 ms, 50 at 23,800 5.13 -> 5.04.  A conditional
-    // node costs four microseconds whether or not it runs, more than the build
-    // of a small system lends: 2,700 atoms 44 us a step with one, 49 with two.
+    // no lists, so on a step that rebuilds it runs beside their build.  A
+    // conditional node costs four microseconds whether or not it runs, more than
+    // the build of a small system lends.  A step with one and with two of them:
+    // 2,700 atoms 50 and 54 us, 10,800 66 and 70, 16,200 84 and 83, 23,800 94 and
+    // 95, 48,600 152 and 152, 64,800 184 and 185, 94,100 257 and 253, 259,200 640
+    // and 636, 473,400 1454 and 1451.
     Nodes head, grid, order, lists, pme, forces, last;
     const bool with_pme = (vv.force_mask & NXM_FORCE_NONBONDED) && plan_.nz;
     e = captured_after(st_, {}, [&] {

@@ -111,10 +111,11 @@ __host__ __device__ __forceinline__ int pair_first(int start, int c) { return (s
 __host__ __device__ __forceinline__ int pair_stride(int stride) { return 2 * stride + 256; }
 
 // Threads per block of the kernels with a thread per atom or term: 256, or 64
-// where that leaves SMs without a block of their own (their FP64 and latency
-// chains then share fewer SMs): integration at 2,700 atoms 8.2 -> 6.5 us, a
-// step at 23,800 92 -> 88 us, an FP64 one 890 -> 832
-inline int thread_block(long long n) { return n >= 2 * 152 * 256 ? 256 : 64; }
+// where 256 give an SM less than two blocks (their FP64 and latency chains then
+// share fewer SMs): integration at 2,700 atoms 8.2 -> 6.5 us, a step at 23,800
+// 92 -> 88 us, an FP64 one 890 -> 832.  From about 50,000 on the two are alike:
+// a step at 48,600 152 and 150, 64,800 186 and 185, 97,200 265 and 266 us.
+inline int thread_block(long long n) { return n >= 2 * kSMs * 256 ? 256 : 64; }
 
 // Context creation: the exclusion sets built on the device
 // (k_exclusions_build.cu).  deg, xdeg, afill and xfill are consecutive runs
