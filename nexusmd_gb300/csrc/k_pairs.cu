@@ -791,8 +791,8 @@ __global__ void __launch_bounds__(W * 32, W <= kHoodWarps ? 2 : 1) k_pairs_mixed
 //    (1 - e)^(-1/2) to second order), and the Ewald terms from polynomials in
 //    r^2 in a table that stays in L1 (nxm_ewald64.cuh): about 40 FP64
 //    instructions per pair, where erfc, exp, sqrt and the divisions took
-//    about 240 per list entry.  23,800 atoms: 5,390 -> 554 us, the FP64 pipe
-//    busy 79% of the kernel's active cycles; 2,700 atoms: 727 -> 92 us.
+//    about 240 per list entry.  23,800 atoms: 5,390 -> 553 us, the FP64 pipe
+//    busy 78% of the kernel's active cycles; 2,700 atoms: 727 -> 92 us.
 // The pair set is decided on the exact r^2 of the reference's list.
 
 constexpr int kWarps64 = 8;

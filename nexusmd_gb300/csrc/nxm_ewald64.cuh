@@ -12,8 +12,8 @@
 // as the cutoffs of the context reach; each is a polynomial of degree 6 about
 // its centre: the Taylor series to degree 13, its higher powers expressed by
 // lower ones (Chebyshev economization), which leaves less than 1e-16 of the
-// term.  Error of a single term against long-precision values, in units of
-// 1e-16, RMS over distances about 0.2, 0.5, 0.8 and 0.99 of a 1 nm cutoff:
+// term.  Error of a single force term against long-precision values, in units
+// of 1e-16, RMS over distances about 0.2, 0.5, 0.8 and 0.99 of a 1 nm cutoff:
 // tolerance 5e-4 1.7, 2.3, 4.3, 4.0 (formed by erfc and exp: 2.6, 4.0, 8.4,
 // 9.8; as a difference throughout: 2.2, 6.2, 60, 650); 1e-19: 2.7, 11, 28, 38
 // (3.9, 16, 43, 53).
